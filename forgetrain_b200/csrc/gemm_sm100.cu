@@ -59,9 +59,10 @@ struct GemmParams {
   int split_from, total_units;
 };
 
-template <int BN, int STAGES, int EPI_BUFS = 1>
+// MT: 128-row blocks of A per tile (1: 128 x BN tiles, 2: 256 x BN tiles)
+template <int BN, int STAGES, int EPI_BUFS = 1, int MT = 1>
 struct GemmSmem {
-  static constexpr int A_BYTES = GEMM_BM * GEMM_BK * 2;
+  static constexpr int A_BYTES = MT * GEMM_BM * GEMM_BK * 2;
   static constexpr int B_BYTES = BN * GEMM_BK * 2;
   static constexpr int STAGE_BYTES = A_BYTES + B_BYTES;
   static constexpr int EPI_BUF_BYTES = 4096 * EPI_BUFS;      // boxes of 32 rows x 128 B
@@ -70,7 +71,9 @@ struct GemmSmem {
   static constexpr int TOTAL = BAR_OFFSET + 512 + 1024;      // + barriers + alignment slack
 };
 
-// `half`: -1 for a whole tile, else which half of the tile's columns this unit covers.
+// `half`: -1 for a whole tile, else which half of the tile this unit covers: of its columns
+// (MT == 1) or of its rows (MT == 2). `mt` counts tiles of MT * 128 rows.
+template <int MT = 1>
 __device__ __forceinline__ void decode_tile(const GemmParams& p, int tile, int& mt, int& nt,
                                             int& kb, int& kn, int& half) {
   half = -1;
@@ -82,10 +85,11 @@ __device__ __forceinline__ void decode_tile(const GemmParams& p, int tile, int& 
   const int per_split = p.m_tiles * p.n_tiles;
   const int ks = tile / per_split;
   const int r = tile - ks * per_split;
-  const int group_sz = GEMM_GROUP_M * p.n_tiles;
+  constexpr int GROUP_M = GEMM_GROUP_M / MT;
+  const int group_sz = GROUP_M * p.n_tiles;
   const int g = r / group_sz;
-  const int first_m = g * GEMM_GROUP_M;
-  const int gm = min(p.m_tiles - first_m, GEMM_GROUP_M);
+  const int first_m = g * GROUP_M;
+  const int gm = min(p.m_tiles - first_m, GROUP_M);
   const int in = r - g * group_sz;
   mt = first_m + in % gm;
   nt = in / gm;
@@ -94,14 +98,77 @@ __device__ __forceinline__ void decode_tile(const GemmParams& p, int tile, int& 
   kn = base + (ks < rem ? 1 : 0);
 }
 
+// One 32 x 64 bf16 box, a row per lane (packed in w[0..31]), through the warp's staging buffer.
+__device__ __forceinline__ void store_piece(const CUtensorMap* tm, int col, int row0,
+                                            const uint32_t* w, uint8_t* sbuf, int lane,
+                                            int& nstores) {
+  if (nstores >= 1) {
+    if (lane == 0) tma_wait_group_read<0>();
+    __syncwarp();
+  }
+#pragma unroll
+  for (int j = 0; j < 8; ++j)
+    *reinterpret_cast<uint4*>(sbuf + lane * 128 + ((j ^ (lane & 7)) << 4)) =
+        make_uint4(w[4 * j], w[4 * j + 1], w[4 * j + 2], w[4 * j + 3]);
+  fence_proxy_async_smem();
+  __syncwarp();
+  if (lane == 0) {
+    tma_store_2d(tm, sbuf, col, row0);
+    tma_commit_group();
+  }
+  ++nstores;
+}
+
+// 256 accumulator columns of this thread's row, scaled and packed. Sixteen columns at a time: with
+// 168 registers for a thread there is no room for more beside the 128 results.
+__device__ __forceinline__ void tmem_ld_packed256(uint32_t taddr, float alpha, uint32_t* w) {
+#pragma unroll
+  for (int c = 0; c < 16; ++c) {
+    uint32_t r[16];
+    tmem_ld16(taddr + c * 16, r);
+    tmem_ld_wait();
+#pragma unroll
+    for (int i = 0; i < 8; ++i)
+      w[c * 8 + i] = pack_bf16x2(__uint_as_float(r[2 * i]) * alpha,
+                                 __uint_as_float(r[2 * i + 1]) * alpha);
+  }
+}
+
+// silu(gate) * up of two packed bf16 pairs, the arithmetic of swiglu_fwd_kernel.
+__device__ __forceinline__ uint32_t swiglu_pair(uint32_t gw, uint32_t uw) {
+  const float g0 = __uint_as_float(gw << 16), g1 = __uint_as_float(gw & 0xffff0000u);
+  const float u0 = __uint_as_float(uw << 16), u1 = __uint_as_float(uw & 0xffff0000u);
+  const float s0 = 1.f / (1.f + __expf(-g0)), s1 = 1.f / (1.f + __expf(-g1));
+  return pack_bf16x2(g0 * s0 * u0, g1 * s1 * u1);
+}
+
 // Epilogue of one 128 x ncols accumulator for one warp: its 32 TMEM lanes (rows row0..row0+31),
 // column half `chalf`. TMEM -> registers -> (alpha, convert) -> swizzled staging buffer ->
 // TMA store / reduce-add. `nstores` counts this warp's bulk groups so the staging buffer is
-// only rewritten after the previous store has read it.
+// only rewritten after the previous store has read it. `release` is called once, when the warp
+// has read its share of the accumulator.
+// WHOLE (tiles of two row blocks, always 256 columns): one warp per TMEM lane quarter drains all
+// columns of an accumulator, and the warps of the other accumulator run beside it. The two
+// accumulators belong to ONE tile, so the first k-step of the next tile waits for each of them
+// right after it was completed: the warp takes all its columns out of TMEM as packed bf16 and
+// releases them before it stores anything.
+template <bool WHOLE, class Release>
 __device__ __forceinline__ void drain_tile(const GemmParams& p, const CUtensorMap* tmD,
                                            uint32_t taddr, int row0, int colbase, int ncols,
-                                           int chalf, uint8_t* sbuf, int lane, int& nstores) {
+                                           int chalf, uint8_t* sbuf, int lane, int& nstores,
+                                           Release release) {
   const bool rows_live = row0 < p.M;
+  if (WHOLE && p.out_mode == OUT_BF16) {
+    uint32_t w[128];
+    tmem_ld_packed256(taddr, p.alpha, w);
+    release();
+#pragma unroll
+    for (int c = 0; c < 4; ++c) {
+      const int col0 = colbase + c * 64;
+      if (col0 < p.N && rows_live) store_piece(tmD, col0, row0, w + c * 32, sbuf, lane, nstores);
+    }
+    return;
+  }
   if (p.out_mode == OUT_BF16) {
 #pragma unroll 1
     for (int c = chalf * (ncols / 128); c < (chalf + 1) * (ncols / 128); ++c) {
@@ -138,7 +205,7 @@ __device__ __forceinline__ void drain_tile(const GemmParams& p, const CUtensorMa
     }
   } else {
 #pragma unroll 1
-    for (int c = chalf * (ncols / 64); c < (chalf + 1) * (ncols / 64); ++c) {
+    for (int c = WHOLE ? 0 : chalf * (ncols / 64); c < (WHOLE ? 8 : (chalf + 1) * (ncols / 64)); ++c) {
       const int col0 = colbase + c * 32;
       if (col0 >= p.N || !rows_live) break;
       uint32_t r[32];
@@ -169,6 +236,7 @@ __device__ __forceinline__ void drain_tile(const GemmParams& p, const CUtensorMa
       ++nstores;
     }
   }
+  release();
 }
 
 // Epilogue of the fused FC1 + SwiGLU tile. The accumulator's columns 0..127 are gate columns
@@ -177,35 +245,21 @@ __device__ __forceinline__ void drain_tile(const GemmParams& p, const CUtensorMa
 // backward pass reads, and act = silu(gate) * up into ACT. The activation is computed from the
 // ROUNDED bf16 gate / up values with the arithmetic of swiglu_fwd_kernel, so it is bitwise the
 // result of running that kernel on Y.
+template <class Release>
 __device__ __forceinline__ void drain_tile_swiglu(const GemmParams& p, const CUtensorMap* tmY,
                                                   const CUtensorMap* tmAct, uint32_t taddr,
                                                   int row0, int n0, int chalf, uint8_t* sbuf,
-                                                  int lane, int& nstores) {
-  if (row0 >= p.M) return;
+                                                  int lane, int& nstores, Release release) {
   const int gcol = n0 + chalf * 64;
-  if (gcol >= p.swiglu_F) return;
+  if (row0 >= p.M || gcol >= p.swiglu_F) {
+    release();
+    return;
+  }
   // Three 64-column stores go through the warp's one staging buffer, each waiting until the
   // previous store has read it. The TMEM load of the up half and the activation arithmetic are
   // placed between the stores so that they run during those reads.
   uint32_t g[32], u[32];   // 64 gate and 64 up values of this thread's row, packed bf16x2
   uint32_t r[64];
-  auto put = [&](const uint32_t* w, const CUtensorMap* tm, int col) {
-    if (nstores >= 1) {
-      if (lane == 0) tma_wait_group_read<0>();
-      __syncwarp();
-    }
-#pragma unroll
-    for (int j = 0; j < 8; ++j)
-      *reinterpret_cast<uint4*>(sbuf + lane * 128 + ((j ^ (lane & 7)) << 4)) =
-          make_uint4(w[4 * j], w[4 * j + 1], w[4 * j + 2], w[4 * j + 3]);
-    fence_proxy_async_smem();
-    __syncwarp();
-    if (lane == 0) {
-      tma_store_2d(tm, sbuf, col, row0);
-      tma_commit_group();
-    }
-    ++nstores;
-  };
   tmem_ld32(taddr + chalf * 64, r);
   tmem_ld32(taddr + chalf * 64 + 32, r + 32);
   tmem_ld_wait();
@@ -214,21 +268,39 @@ __device__ __forceinline__ void drain_tile_swiglu(const GemmParams& p, const CUt
     g[i] = pack_bf16x2(__uint_as_float(r[2 * i]) * p.alpha, __uint_as_float(r[2 * i + 1]) * p.alpha);
   tmem_ld32(taddr + 128 + chalf * 64, r);
   tmem_ld32(taddr + 128 + chalf * 64 + 32, r + 32);
-  put(g, tmY, gcol);
+  store_piece(tmY, gcol, row0, g, sbuf, lane, nstores);
   tmem_ld_wait();
 #pragma unroll
   for (int i = 0; i < 32; ++i)
     u[i] = pack_bf16x2(__uint_as_float(r[2 * i]) * p.alpha, __uint_as_float(r[2 * i + 1]) * p.alpha);
-  put(u, tmY, p.swiglu_F + gcol);
+  release();
+  store_piece(tmY, p.swiglu_F + gcol, row0, u, sbuf, lane, nstores);
 #pragma unroll
-  for (int i = 0; i < 32; ++i) {
-    const uint32_t gw = g[i], uw = u[i];
-    const float g0 = __uint_as_float(gw << 16), g1 = __uint_as_float(gw & 0xffff0000u);
-    const float u0 = __uint_as_float(uw << 16), u1 = __uint_as_float(uw & 0xffff0000u);
-    const float s0 = 1.f / (1.f + __expf(-g0)), s1 = 1.f / (1.f + __expf(-g1));
-    g[i] = pack_bf16x2(g0 * s0 * u0, g1 * s1 * u1);
+  for (int i = 0; i < 32; ++i) g[i] = swiglu_pair(g[i], u[i]);
+  store_piece(tmAct, gcol, row0, g, sbuf, lane, nstores);
+}
+
+// The same for a tile of two row blocks (see WHOLE at drain_tile): one warp drains the gate and
+// the up columns of its 32 rows, all of them into registers first.
+template <class Release>
+__device__ __forceinline__ void drain_tile_swiglu_whole(const GemmParams& p,
+                                                        const CUtensorMap* tmY,
+                                                        const CUtensorMap* tmAct, uint32_t taddr,
+                                                        int row0, int n0, uint8_t* sbuf, int lane,
+                                                        int& nstores, Release release) {
+  uint32_t w[128];   // 128 gate, then 128 up values, packed bf16x2
+  tmem_ld_packed256(taddr, p.alpha, w);
+  release();
+  if (row0 >= p.M) return;
+#pragma unroll
+  for (int c = 0; c < 2; ++c) {
+    const int gcol = n0 + c * 64;
+    store_piece(tmY, gcol, row0, w + c * 32, sbuf, lane, nstores);
+#pragma unroll
+    for (int i = 0; i < 32; ++i) w[c * 32 + i] = swiglu_pair(w[c * 32 + i], w[64 + c * 32 + i]);
+    store_piece(tmY, p.swiglu_F + gcol, row0, w + 64 + c * 32, sbuf, lane, nstores);
+    store_piece(tmAct, gcol, row0, w + c * 32, sbuf, lane, nstores);
   }
-  put(g, tmAct, gcol);
 }
 
 // Epilogue of the fused FC2 dgrad + SwiGLU backward kernel (EPI_SWIGLU_BWD), one warp's share.
@@ -260,14 +332,21 @@ __device__ __forceinline__ void swiglu_bwd_tile_info(const GemmParams& p, int ti
   nvalid = row0 < p.M ? max(0, min(ncols / 64, left)) : 0;
 }
 
-template <int BN, int STAGES, int EPI = EPI_PLAIN>
+// MT == 2 (256 x 256 tiles): the two TMEM accumulators are the two 128-row blocks of one tile, which
+// share the B operand of a k-step. A 128 x 256 tile moves 48 KB through TMA and shared memory per
+// 512 tensor cycles (96 B per cycle and SM, above the ~75 that arrive from L2), a 256 x 256 tile
+// 64 KB per 1024 cycles. `it` counts accumulators, so that buffer and phase of block s of a unit are
+// (it + s) & 1 and ((it + s) >> 1) & 1 in the issuing and in the epilogue warps alike.
+template <int BN, int STAGES, int EPI = EPI_PLAIN, int MT = 1>
 __global__ void __launch_bounds__(GEMM_THREADS, 1)
 gemm_bf16_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUtensorMap tmB,
                  const __grid_constant__ CUtensorMap tmD, const __grid_constant__ CUtensorMap tmD2,
                  const GemmParams p) {
   constexpr bool SWIGLU = EPI == EPI_SWIGLU_FWD;
   static_assert(EPI == EPI_PLAIN || BN == 256, "the fused SwiGLU epilogues are built for 256-column tiles");
-  using L = GemmSmem<BN, STAGES, EPI == EPI_SWIGLU_BWD ? 2 : 1>;
+  static_assert(MT == 1 || (MT == 2 && BN == 256 && EPI != EPI_SWIGLU_BWD),
+                "two row blocks: 256-column tiles, and one staging buffer per epilogue warp");
+  using L = GemmSmem<BN, STAGES, EPI == EPI_SWIGLU_BWD ? 2 : 1, MT>;
   extern __shared__ uint8_t smem_raw[];
   uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) &
                                              ~static_cast<uintptr_t>(1023));
@@ -291,7 +370,7 @@ gemm_bf16_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant_
     }
     for (int b = 0; b < 2; ++b) {
       mbar_init(&tfull_bar[b], 1);
-      mbar_init(&tempty_bar[b], GEMM_EPI_WARPS);
+      mbar_init(&tempty_bar[b], MT == 2 ? GEMM_EPI_WARPS / 2 : GEMM_EPI_WARPS);
     }
     for (int w = 0; w < 2 * GEMM_EPI_WARPS; ++w) mbar_init(&ybar[w], 1);
     *abort_flag = 0;
@@ -315,20 +394,25 @@ gemm_bf16_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant_
   if (warp == 0 || warp == GEMM_PRODUCER_WARP2) {
     // ------------------------------ TMA producers ------------------------------
     // Lane l issues box l of a stage: A is one 128-row box (K-major) or two 64 x 64 boxes
-    // (MN-major); B is BN/128 boxes of 128 rows or BN/64 boxes of 64 x 64.
+    // (MN-major) per row block; B is BN/128 boxes of 128 rows or BN/64 boxes of 64 x 64.
     const int pid = warp == 0 ? 0 : 1;
-    const int nA = p.a_mn ? GEMM_BM / 64 : 1;
+    const int nA = (p.a_mn ? GEMM_BM / 64 : 1) * MT;
     const int nB = p.b_mn ? BN / 64 : BN / 128;
     if (lane < nA + nB) {
       int stage = 0;
       uint32_t phase = 0;
       for (int tile = blockIdx.x; tile < total_tiles; tile += gridDim.x) {
         int mt, nt, kb, kn, half;
-        decode_tile(p, tile, mt, nt, kb, kn, half);
-        // a half tile loads only its half of the B boxes, into the start of the B buffer
-        const int nBt = half < 0 ? nB : nB / 2;
-        const int jb0 = half <= 0 ? 0 : nB / 2;
-        const uint32_t tx = L::A_BYTES + (half < 0 ? L::B_BYTES : L::B_BYTES / 2);
+        decode_tile<MT>(p, tile, mt, nt, kb, kn, half);
+        // a half tile loads only its half of the B boxes (MT == 1) or of the A boxes (MT == 2),
+        // into the start of that buffer
+        const bool halfA = MT == 2 && half >= 0, halfB = MT == 1 && half >= 0;
+        const int nAt = halfA ? nA / 2 : nA;
+        const int nBt = halfB ? nB / 2 : nB;
+        const int jb0 = halfB && half > 0 ? nB / 2 : 0;
+        const int row0 = mt * (MT * GEMM_BM) + (halfA && half > 0 ? GEMM_BM : 0);
+        const uint32_t tx = (halfA ? L::A_BYTES / 2 : L::A_BYTES) +
+                            (halfB ? L::B_BYTES / 2 : L::B_BYTES);
         for (int ki = kb; ki < kb + kn; ++ki) {
           if ((stage & 1) == pid) {
             mbar_wait(&empty_bar[stage], phase ^ 1, abort_flag, p.status, FT_ERR_WAIT_EMPTY);
@@ -336,11 +420,14 @@ gemm_bf16_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant_
             uint8_t* sB = sA + L::A_BYTES;
             if (lane == 0) mbar_expect_tx(&full_bar[stage], tx);
             if (lane < nA) {
-              if (!p.a_mn)
-                tma_load_2d(sA, &tmA, &full_bar[stage], ki * GEMM_BK, mt * GEMM_BM);
-              else
-                tma_load_2d(sA + lane * 8192, &tmA, &full_bar[stage], mt * GEMM_BM + lane * 64,
-                            ki * GEMM_BK);
+              if (lane < nAt) {
+                if (!p.a_mn)
+                  tma_load_2d(sA + lane * 16384, &tmA, &full_bar[stage], ki * GEMM_BK,
+                              row0 + lane * GEMM_BM);
+                else
+                  tma_load_2d(sA + lane * 8192, &tmA, &full_bar[stage], row0 + lane * 64,
+                              ki * GEMM_BK);
+              }
             } else if (lane - nA < nBt) {
               const int j = lane - nA;           // slot in the B buffer; jb0 + j: box of the tile
               if (SWIGLU)   // box 0: 128 gate rows, box 1: the 128 up rows of the same columns
@@ -386,7 +473,36 @@ gemm_bf16_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant_
       int it = 0;
       for (int tile = blockIdx.x; tile < total_tiles; tile += gridDim.x, ++it) {
         int mt, nt, kb, kn, half;
-        decode_tile(p, tile, mt, nt, kb, kn, half);
+        decode_tile<MT>(p, tile, mt, nt, kb, kn, half);
+        if constexpr (MT == 2) {
+          const int blocks = half < 0 ? 2 : 1;
+          for (int ki = 0; ki < kn; ++ki) {
+            mbar_wait(&full_bar[stage], phase, abort_flag, p.status, FT_ERR_WAIT_FULL);
+            const uint32_t sA = smem_base + stage * L::STAGE_BYTES;
+            const uint32_t b_lo = smem_desc_lo(sA + L::A_BYTES, b_lbo);
+            for (int s = 0; s < blocks; ++s) {
+              const int buf = (it + s) & 1;
+              if (ki == 0)
+                mbar_wait(&tempty_bar[buf], (((it + s) >> 1) & 1) ^ 1, abort_flag, p.status,
+                          FT_ERR_WAIT_TMEM_EMPTY);
+              tc_fence_after();
+              if (elect_one_sync()) {
+                const uint32_t tmem_d = tmem_base + buf * BN;
+                const uint32_t a_lo = smem_desc_lo(sA + s * 16384, a_lbo);
+                umma_ss_lo_dyn(tmem_d, a_lo, b_lo, idesc_full, ki > 0 ? 1u : 0u);
+#pragma unroll
+                for (int kk = 1; kk < GEMM_BK / 16; ++kk)
+                  umma_ss_lo<1>(tmem_d, a_lo + kk * a_kstep, b_lo + kk * b_kstep, idesc_full);
+                if (s == blocks - 1) umma_commit(&empty_bar[stage]);
+                if (ki == kn - 1) umma_commit(&tfull_bar[buf]);
+              }
+              __syncwarp();
+            }
+            if (++stage == STAGES) { stage = 0; phase ^= 1; }
+          }
+          it += blocks - 1;   // the loop header counts the other one
+          continue;
+        }
         const uint32_t idesc = half < 0 ? idesc_full : idesc_half;
         const int buf = it & 1;
         const uint32_t acc_phase = (it >> 1) & 1;
@@ -416,7 +532,8 @@ gemm_bf16_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant_
   } else {
     // ------------------------------ epilogue ------------------------------
     const int q = warp & 3;             // TMEM lane quarter this warp may access
-    const int chalf = (warp - 2) >> 2;  // which half of the tile's columns this warp drains
+    const int chalf = (warp - 2) >> 2;  // which half of the tile's columns (MT == 2: which of the
+                                        // two accumulators) this warp drains
     uint8_t* my_epi = epi_base + (warp - 2) * L::EPI_BUF_BYTES;
     int it = 0;
     int nstores = 0;
@@ -541,23 +658,35 @@ gemm_bf16_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant_
         if (lane == 0) mbar_arrive(&tempty_bar[buf]);
       }
     } else {
-    for (int tile = blockIdx.x; tile < total_tiles; tile += gridDim.x, ++it) {
+    for (int tile = blockIdx.x; tile < total_tiles; tile += gridDim.x) {
       int mt, nt, kb, kn, half;
-      decode_tile(p, tile, mt, nt, kb, kn, half);
-      const int buf = it & 1;
-      const uint32_t acc_phase = (it >> 1) & 1;
-      mbar_wait(&tfull_bar[buf], acc_phase, abort_flag, p.status, FT_ERR_WAIT_TMEM_FULL);
-      tc_fence_after();
-      const uint32_t taddr = tmem_base + (static_cast<uint32_t>(q * 32) << 16) + buf * BN;
-      const int row0 = mt * GEMM_BM + q * 32;
-      if (SWIGLU)
-        drain_tile_swiglu(p, &tmD, &tmD2, taddr, row0, nt * 128, chalf, my_epi, lane, nstores);
-      else
-        drain_tile(p, &tmD, taddr, row0, nt * BN + (half > 0 ? BN / 2 : 0),
-                   half < 0 ? BN : BN / 2, chalf, my_epi, lane, nstores);
-      tc_fence_before();
-      __syncwarp();
-      if (lane == 0) mbar_arrive(&tempty_bar[buf]);
+      decode_tile<MT>(p, tile, mt, nt, kb, kn, half);
+      const int blocks = MT == 2 && half < 0 ? 2 : 1;
+      for (int s = 0; s < blocks; ++s, ++it) {
+        const int buf = it & 1;
+        if (MT == 2 && buf != chalf) continue;   // the other four warps drain that accumulator
+        const uint32_t acc_phase = (it >> 1) & 1;
+        mbar_wait(&tfull_bar[buf], acc_phase, abort_flag, p.status, FT_ERR_WAIT_TMEM_FULL);
+        tc_fence_after();
+        const uint32_t taddr = tmem_base + (static_cast<uint32_t>(q * 32) << 16) + buf * BN;
+        const int row0 = (mt * MT + (MT == 2 && half > 0 ? 1 : s)) * GEMM_BM + q * 32;
+        auto release = [&]() {
+          tc_fence_before();
+          __syncwarp();
+          if (lane == 0) mbar_arrive(&tempty_bar[buf]);
+        };
+        if (SWIGLU && MT == 2)
+          drain_tile_swiglu_whole(p, &tmD, &tmD2, taddr, row0, nt * 128, my_epi, lane, nstores,
+                                  release);
+        else if (SWIGLU)
+          drain_tile_swiglu(p, &tmD, &tmD2, taddr, row0, nt * 128, chalf, my_epi, lane, nstores,
+                            release);
+        else
+          drain_tile<MT == 2>(p, &tmD, taddr, row0,
+                              nt * BN + (MT == 1 && half > 0 ? BN / 2 : 0),
+                              MT == 2 || half < 0 ? BN : BN / 2, chalf, my_epi, lane, nstores,
+                              release);
+      }
     }
     }
     if (lane == 0) tma_wait_group<0>();
@@ -764,10 +893,11 @@ gemm_pair_bf16_kernel(const __grid_constant__ CUtensorMap tmA,
       tc_fence_after();
       const uint32_t taddr = tmem_base + (static_cast<uint32_t>(q * 32) << 16) + buf * BN;
       const int row0 = mt * 256 + static_cast<int>(rank) * 128 + q * 32;
-      drain_tile(p, &tmD, taddr, row0, nt * BN, BN, chalf, my_epi, lane, nstores);
-      tc_fence_before();
-      __syncwarp();
-      if (lane == 0) mbar_arrive_cluster(tempty0 + buf * 8);
+      drain_tile<false>(p, &tmD, taddr, row0, nt * BN, BN, chalf, my_epi, lane, nstores, [&]() {
+        tc_fence_before();
+        __syncwarp();
+        if (lane == 0) mbar_arrive_cluster(tempty0 + buf * 8);
+      });
     }
     if (lane == 0) tma_wait_group<0>();
     __syncwarp();
@@ -857,14 +987,14 @@ static int num_sms() {
   return g_num_sms;
 }
 
-template <int BN, int STAGES, int EPI = EPI_PLAIN>
+template <int BN, int STAGES, int EPI = EPI_PLAIN, int MT = 1>
 static int launch_gemm(const CUtensorMap& tmA, const CUtensorMap& tmB, const CUtensorMap& tmD,
                        const CUtensorMap& tmD2, const GemmParams& p, int max_ctas,
                        cudaStream_t stream) {
-  using L = GemmSmem<BN, STAGES, EPI == EPI_SWIGLU_BWD ? 2 : 1>;
+  using L = GemmSmem<BN, STAGES, EPI == EPI_SWIGLU_BWD ? 2 : 1, MT>;
   static bool attr_set = false;
   if (!attr_set) {
-    cudaError_t e = cudaFuncSetAttribute(gemm_bf16_kernel<BN, STAGES, EPI>,
+    cudaError_t e = cudaFuncSetAttribute(gemm_bf16_kernel<BN, STAGES, EPI, MT>,
                                          cudaFuncAttributeMaxDynamicSharedMemorySize, L::TOTAL);
     if (e != cudaSuccess) return -10;
     attr_set = true;
@@ -872,9 +1002,72 @@ static int launch_gemm(const CUtensorMap& tmA, const CUtensorMap& tmB, const CUt
   const int total = p.total_units;
   int grid = total < max_ctas ? total : max_ctas;
   if (grid < 1) grid = 1;
-  gemm_bf16_kernel<BN, STAGES, EPI>
+  gemm_bf16_kernel<BN, STAGES, EPI, MT>
       <<<grid, GEMM_THREADS, L::TOTAL, stream>>>(tmA, tmB, tmD, tmD2, p);
   return cudaGetLastError() == cudaSuccess ? 0 : -11;
+}
+
+// Tail of the schedule: when the last wave is at most half full, its tiles are cut in two, so that
+// twice as many CTAs work on it. Shapes of the 0.5B model at 16384 tokens with 128 x 256 tiles: the
+// attention-output and FC2-forward GEMMs have 512 tiles = 3.46 waves of 148, QKV 640 = 4.32.
+static void cut_tail(GemmParams& p, int max_ctas) {
+  const int total = p.total_units;
+  if (max_ctas < 2) return;
+  const int rem = total % max_ctas;
+  if (rem > 0 && 2 * rem <= max_ctas) {
+    p.split_from = total - rem;
+    p.total_units = total + rem;
+  }
+}
+
+static int auto_splitk(int tiles, int k_iters, int max_ctas) {
+  if (tiles >= max_ctas) return 1;
+  int splitk = max_ctas / tiles;
+  const int max_by_k = k_iters / 8 > 0 ? k_iters / 8 : 1;
+  if (splitk > max_by_k) splitk = max_by_k;
+  if (splitk > 16) splitk = 16;
+  return splitk;
+}
+
+struct GemmPlan {
+  int mt, splitk;
+};
+
+// Tile height and split of the reduction for 256-column tiles, by the estimated length of the
+// schedule. Unit: a hundredth of what one k-step of a 128 x 256 tile costs a CTA (about 400 ns under
+// load). Measured over T = 256 .. 16384 tokens with the shapes of the 0.5B and 8B layers, operands
+// rotated through more than L2, back to back in a graph (us, 128 x 256 -> 256 x 256 tiles):
+//   fc1 fwd   16384 x 8192 x 1024   214 -> 197      fc1 wgrad  8192 x 1024 x 16384  211 -> 185
+//   fc2 fwd   16384 x 1024 x 4096   104 -> 99       8B qkv fwd  4096 x 4608 x 4096  111 -> 101
+//   8B fc2 fwd 4096 x 4096 x 16384  414 -> 368      8B wo wgrad 8192 x 4096 x 4096  215 -> 194
+//   wo fwd    16384 x 1024 x 1024   31.0 -> 31.2    qkv fwd    16384 x 1280 x 1024  37.9 -> 40.0
+//   fc2 fwd    4096 x 1024 x 4096   30.9 -> 38.4    8B qkv fwd  1024 x 4608 x 4096  30.8 -> 37.5
+// The last four are short of tiles: a 256 x 256 tile costs 1.75 of a 128 x 256 one, a half of it 1.2
+// (a half of the small one 0.8), and its epilogue is exposed for about 2.5 (fp32: 4) k-steps. A
+// split costs the memset and the reduce-adds, about 16 k-steps (10 without the memset): QKV wgrad
+// at 1024 tokens 13.1 us split in two, 10.2 whole.
+static GemmPlan pick_plan(int M, int N, int k_iters, bool f32, int accumulate, int max_ctas) {
+  GemmPlan best{1, 1};
+  long best_cost = 0;
+  for (int mt = 1; mt <= 2; ++mt) {
+    const long tiles = static_cast<long>((M + GEMM_BM * mt - 1) / (GEMM_BM * mt)) * ((N + 255) / 256);
+    const int max_split = f32 && tiles < max_ctas ? auto_splitk(static_cast<int>(tiles), k_iters, max_ctas) : 1;
+    for (int s = 1; s <= max_split; ++s) {
+      const long units = tiles * s, waves = units / max_ctas, rem = units % max_ctas;
+      const long k = (k_iters + s - 1) / s;
+      const long whole = mt == 2 ? 175 * k + (f32 ? 400 : 250) : 100 * k;
+      const long half = mt == 2 ? 120 * k + 250 : 80 * k;
+      long cost = waves * whole;
+      if (rem) cost += s == 1 && 2 * rem <= max_ctas ? half : whole;
+      if (s > 1) cost += accumulate ? 1000 : 1650;
+      if (mt == 2) cost += cost / 50;   // a tie stays with the smaller tile
+      if (best_cost == 0 || cost < best_cost) {
+        best_cost = cost;
+        best = GemmPlan{mt, s};
+      }
+    }
+  }
+  return best;
 }
 
 #ifdef FT_BUILD_PAIR_GEMM
@@ -903,6 +1096,7 @@ static int launch_gemm_pair(const CUtensorMap& tmA, const CUtensorMap& tmB,
 // Tile selection, per shape class (what the rules below resolve to for the two model families at
 // their benchmark token counts; TFLOP/s measured on a B200 at boost clock, cuBLAS in brackets):
 //
+// (Figures of 128 x 256 tiles; which shapes take 256 x 256 ones is pick_plan's rule.)
 //   shape (M x N x K)                 tile      split / tail              fwd    dgrad  wgrad
 //   0.5B qkv      16384 x 1280 x 1024 128x256   tail: 48 tiles halved      975    999    819  (1135/1076/893)
 //   0.5B attn_out 16384 x 1024 x 1024 128x256   tail: 68 tiles halved      932    932    780  ( 959/1015/818)
@@ -921,7 +1115,7 @@ static int launch_gemm_pair(const CUtensorMap& tmA, const CUtensorMap& tmB,
 //   a_mn == 0: A is stored [M][lda] (reduction index contiguous); a_mn == 1: A is stored
 //   [K][lda] (row index contiguous). Same for B with N. out_dtype: 0 bf16, 1 fp32.
 //   accumulate != 0 (fp32 only): D += result. splitk <= 0 picks a split automatically
-//   (fp32 only); bn in {0 (auto), 128, 256}. All leading dimensions in elements; every base
+//   (fp32 only); bn in {0 (auto), 128, 256: one 128 x bn tile, 512: a 256 x 256 tile per CTA}. All leading dimensions in elements; every base
 //   pointer 16-byte aligned and every leading dimension a multiple of 8 (bf16) / 4 (fp32).
 extern "C" int ft_gemm_bf16(const void* A, const void* B, void* D, int M, int N, int K, int lda,
                             int ldb, int ldd, int a_mn, int b_mn, int out_dtype, int accumulate,
@@ -933,24 +1127,19 @@ extern "C" int ft_gemm_bf16(const void* A, const void* B, void* D, int M, int N,
   const int sms = num_sms();
   if (max_ctas <= 0 || max_ctas > sms) max_ctas = sms;
   const int k_iters = (K + GEMM_BK - 1) / GEMM_BK;
-  // bn: 128 / 256 = one CTA per 128 x bn tile.
-  if (bn != 128 && bn != 256) bn = (N <= 128) ? 128 : 256;
-  constexpr bool pair = false;
-  const int bm = GEMM_BM;
-  const int m_tiles = (M + bm - 1) / bm;
-  const int n_tiles = (N + bn - 1) / bn;
   if (out_dtype == 0) splitk = 1;
-  if (splitk <= 0) {
-    const int tiles = m_tiles * n_tiles;
-    splitk = 1;
-    const int units = pair ? max_ctas / 2 : max_ctas;
-    if (tiles < units) {
-      splitk = units / tiles;
-      const int max_by_k = k_iters / 8 > 0 ? k_iters / 8 : 1;
-      if (splitk > max_by_k) splitk = max_by_k;
-      if (splitk > 16) splitk = 16;
-    }
+  int mt = bn == 512 ? 2 : 1;
+  const bool pick = bn != 128 && bn != 256 && bn != 512 && N > 128 && (out_dtype == 0 || splitk <= 0);
+  if (bn == 512) bn = 256;
+  if (bn != 128 && bn != 256) bn = (N <= 128) ? 128 : 256;
+  if (pick) {
+    const GemmPlan plan = pick_plan(M, N, k_iters, out_dtype == 1, accumulate, max_ctas);
+    mt = plan.mt;
+    splitk = plan.splitk;
   }
+  const int m_tiles = (M + GEMM_BM * mt - 1) / (GEMM_BM * mt);
+  const int n_tiles = (N + bn - 1) / bn;
+  if (splitk <= 0) splitk = auto_splitk(m_tiles * n_tiles, k_iters, max_ctas);
   if (splitk > k_iters) splitk = k_iters;
   if (splitk < 1) splitk = 1;
 
@@ -962,22 +1151,8 @@ extern "C" int ft_gemm_bf16(const void* A, const void* B, void* D, int M, int N,
   p.m_tiles = m_tiles; p.n_tiles = n_tiles; p.k_iters = k_iters;
   p.status = status;
   p.swiglu_F = 0;
-  {
-    // Tail of the schedule: when the last wave is at most half full, its tiles are cut in two
-    // (128 x 128 halves on twice as many CTAs). Shapes of the 0.5B model at 16384 tokens: the
-    // attention-output, FC2-forward and FC1-dgrad GEMMs have 512 tiles = 3.46 waves of 148, the
-    // QKV forward 640 = 4.32; a half tile costs about 0.6 of a whole one.
-    const int total = m_tiles * n_tiles * splitk;
-    p.split_from = total;
-    p.total_units = total;
-    if (bn == 256 && splitk == 1 && max_ctas >= 2) {
-      const int rem = total % max_ctas;
-      if (rem > 0 && 2 * rem <= max_ctas) {
-        p.split_from = total - rem;
-        p.total_units = total + rem;
-      }
-    }
-  }
+  p.split_from = p.total_units = m_tiles * n_tiles * splitk;
+  if (bn == 256 && splitk == 1) cut_tail(p, max_ctas);
   if (out_dtype == 0) p.out_mode = OUT_BF16;
   else p.out_mode = (accumulate || splitk > 1) ? OUT_F32_ADD : OUT_F32;
   if (out_dtype == 1 && !accumulate && splitk > 1) {
@@ -998,6 +1173,7 @@ extern "C" int ft_gemm_bf16(const void* A, const void* B, void* D, int M, int N,
   else                rc = get_tmap_2d(&tmD, D, 4, M, N, ldd, 32, 32);
   if (rc) return -6;
 
+  if (mt == 2) return launch_gemm<256, 3, EPI_PLAIN, 2>(tmA, tmB, tmD, tmD, p, max_ctas, stream);
   if (bn == 256) return launch_gemm<256, 4>(tmA, tmB, tmD, tmD, p, max_ctas, stream);
   return launch_gemm<128, 6>(tmA, tmB, tmD, tmD, p, max_ctas, stream);
 }
@@ -1014,23 +1190,31 @@ extern "C" int ft_gemm_swiglu_bf16(const void* A, const void* W, void* Y, void* 
   if (F % 128) return -2;
   const int sms = num_sms();
   if (max_ctas <= 0 || max_ctas > sms) max_ctas = sms;
+  // Two row blocks from K = 2048 on: 8B FC1 at 8192 tokens 1.75 -> 1.53 ms, at 4096 tokens 788 -> 751
+  // us. At K = 1024 a tile's main loop is shorter than the three stores and the activation of its
+  // 256 x 128 outputs take the four warps of an accumulator: 253 -> 263 us at 16384 tokens.
+  const int k_iters = (K + GEMM_BK - 1) / GEMM_BK;
+  const int mt = k_iters >= 32 && pick_plan(M, 2 * F, k_iters, false, 0, max_ctas).mt == 2 ? 2 : 1;
   GemmParams p;
   p.M = M; p.N = 2 * F; p.K = K;
   p.a_mn = 0; p.b_mn = 0;
   p.out_mode = OUT_BF16;
   p.alpha = alpha;
   p.splitk = 1;
-  p.m_tiles = (M + GEMM_BM - 1) / GEMM_BM;
+  p.m_tiles = (M + GEMM_BM * mt - 1) / (GEMM_BM * mt);
   p.n_tiles = F / 128;
-  p.k_iters = (K + GEMM_BK - 1) / GEMM_BK;
+  p.k_iters = k_iters;
   p.status = status;
   p.swiglu_F = F;
   p.split_from = p.total_units = p.m_tiles * p.n_tiles;
+  if (mt == 2) cut_tail(p, max_ctas);
   CUtensorMap tmA, tmB, tmY, tmAct;
   if (get_tmap_2d(&tmA, A, 2, M, K, lda, GEMM_BM, GEMM_BK)) return -4;
   if (get_tmap_2d(&tmB, W, 2, 2 * static_cast<uint64_t>(F), K, ldw, 128, GEMM_BK)) return -5;
   if (get_tmap_2d(&tmY, Y, 2, M, 2 * static_cast<uint64_t>(F), ldy, 32, 64)) return -6;
   if (get_tmap_2d(&tmAct, ACT, 2, M, F, ldact, 32, 64)) return -6;
+  if (mt == 2)
+    return launch_gemm<256, 3, EPI_SWIGLU_FWD, 2>(tmA, tmB, tmY, tmAct, p, max_ctas, stream);
   return launch_gemm<256, 4, EPI_SWIGLU_FWD>(tmA, tmB, tmY, tmAct, p, max_ctas, stream);
 }
 
@@ -1058,13 +1242,8 @@ extern "C" int ft_gemm_swiglu_bwd_bf16(const void* DY, const void* W2, const voi
   p.k_iters = (K + GEMM_BK - 1) / GEMM_BK;
   p.status = status;
   p.swiglu_F = F;
-  const int total = p.m_tiles * p.n_tiles;
-  p.split_from = p.total_units = total;
-  const int rem = total % max_ctas;
-  if (max_ctas >= 2 && rem > 0 && 2 * rem <= max_ctas) {
-    p.split_from = total - rem;
-    p.total_units = total + rem;
-  }
+  p.split_from = p.total_units = p.m_tiles * p.n_tiles;
+  cut_tail(p, max_ctas);
   CUtensorMap tmA, tmB, tmD, tmY;
   if (get_tmap_2d(&tmA, DY, 2, M, K, lddy, GEMM_BM, GEMM_BK)) return -4;
   if (get_tmap_2d(&tmB, W2, 2, K, F, ldw, GEMM_BK, 64)) return -5;
