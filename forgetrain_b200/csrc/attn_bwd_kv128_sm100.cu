@@ -17,6 +17,7 @@
 // TMEM columns: [0,64) S^T, [64,128) dP^T, [128,256) dV, [256,384) dK, [384,448) dQ^T,
 // [448,480) P^T, [480,512) dS^T. Work decomposition, statistics (negated lse2 / delta), the fp32
 // accumulator and the conversion pass are those of attn_bwd_sm100.cu.
+#include "launch.h"
 #include "ptx.cuh"
 #include "tma_host.h"
 
@@ -63,6 +64,7 @@ fa_bwd_kv128_kernel(const __grid_constant__ CUtensorMap tm_kv,    // qkv, boxes 
                     const __grid_constant__ CUtensorMap tm_do,    // dout, boxes of 64 rows x 64 cols
                     const __grid_constant__ CUtensorMap tm_acc,   // accumulator, 32 x 32 fp32 boxes
                     const FaBwd128Params p) {
+  pdl_trigger();
   using L = FaBwd128Smem;
   constexpr int D = FB128_D, QS = FB128_QS;
   extern __shared__ uint8_t smem_raw[];
@@ -139,6 +141,7 @@ fa_bwd_kv128_kernel(const __grid_constant__ CUtensorMap tm_kv,    // qkv, boxes 
   tc_fence_before();
   __syncthreads();
   tc_fence_after();
+  pdl_wait();
   const uint32_t tmem_base = *tmem_slot;
   const uint32_t tm_S = tmem_base;
   const uint32_t tm_dP = tmem_base + 64;
@@ -478,7 +481,7 @@ int launch_fa_bwd_kv128(const CUtensorMap& tkv, const CUtensorMap& tq, const CUt
   p.lse2 = neg_lse2; p.delta = neg_delta; p.acc = acc;
   p.status = status;
   const int grid = (S / FB128_KV) * batch * n_groups * (g / hpc);
-  fa_bwd_kv128_kernel<<<grid, FB128_THREADS, L::TOTAL, st>>>(tkv, tq, tdo, tacc, p);
+  launch_pdl(fa_bwd_kv128_kernel, grid, FB128_THREADS, L::TOTAL, st, tkv, tq, tdo, tacc, p);
   return cudaGetLastError() == cudaSuccess ? 0 : -11;
 }
 

@@ -20,6 +20,7 @@
 // TMEM columns: [0,128) S^T / dP^T, [128,192) dV, [192,256) dK, [256,320) dQ, [320,384) P^T,
 // [384,448) dS^T. Work decomposition, producer, dQ / dK / dV drain and the fp32 accumulator are
 // those of attn_bwd_sm100.cu.
+#include "launch.h"
 #include "ptx.cuh"
 #include "tma_host.h"
 
@@ -66,6 +67,7 @@ template <int QS, int NDS>
 __global__ void __launch_bounds__(FABK_THREADS, 1)
 fa_bwd_kv_kernel(const __grid_constant__ CUtensorMap tm_qkv, const __grid_constant__ CUtensorMap tm_do,
                  const __grid_constant__ CUtensorMap tm_acc, const FaBwdParams p) {
+  pdl_trigger();
   using L = FaBwdKvSmem<QS, NDS>;
   constexpr int D = FABK_D;
   extern __shared__ uint8_t smem_raw[];
@@ -143,6 +145,7 @@ fa_bwd_kv_kernel(const __grid_constant__ CUtensorMap tm_qkv, const __grid_consta
   tc_fence_before();
   __syncthreads();
   tc_fence_after();
+  pdl_wait();
   const uint32_t tmem_base = *tmem_slot;
   const uint32_t tm_SdP = tmem_base;
   const uint32_t tm_dV = tmem_base + 128;
@@ -485,7 +488,7 @@ int launch_fa_bwd_kv64(const CUtensorMap& tq, const CUtensorMap& tdo, const CUte
   p.lse2 = neg_lse2; p.delta = neg_delta; p.acc = acc;
   p.status = status;
   const int grid = (S / FABK_BLK) * batch * n_groups * (g / hpc);
-  fa_bwd_kv_kernel<3, 1><<<grid, FABK_THREADS, L::TOTAL, st>>>(tq, tdo, tacc, p);
+  launch_pdl(fa_bwd_kv_kernel<3, 1>, grid, FABK_THREADS, L::TOTAL, st, tq, tdo, tacc, p);
   return cudaGetLastError() == cudaSuccess ? 0 : -11;
 }
 

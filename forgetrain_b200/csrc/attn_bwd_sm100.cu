@@ -22,6 +22,7 @@
 // (ops/attention/flash_attn_dsl/flash_bwd.py:243-3373).
 #include <stdlib.h>
 
+#include "launch.h"
 #include "ptx.cuh"
 #include "tma_host.h"
 
@@ -81,6 +82,7 @@ template <int D, int QS, int NP, int NDS, int NST>
 __global__ void __launch_bounds__(FAB_THREADS, 1)
 fa_bwd_kernel(const __grid_constant__ CUtensorMap tm_qkv, const __grid_constant__ CUtensorMap tm_do,
               const __grid_constant__ CUtensorMap tm_acc, const FaBwdParams p) {
+  pdl_trigger();
   using L = FaBwdSmem<D, QS, NP, NDS, NST>;
   // head_dim 128 fills all 512 TMEM columns with S, dP, dV and dK, so dQ has to share the
   // columns of dP. The step is then split: S of step n+1 is issued as soon as S of step n is in
@@ -159,6 +161,7 @@ fa_bwd_kernel(const __grid_constant__ CUtensorMap tm_qkv, const __grid_constant_
   tc_fence_before();
   __syncthreads();
   tc_fence_after();
+  pdl_wait();
   const uint32_t tmem_base = *tmem_slot;
   const uint32_t tm_St = tmem_base;
   const uint32_t tm_dPt = tmem_base + 128;
@@ -562,6 +565,8 @@ __global__ void fa_bwd_pre_kernel(const __nv_bfloat16* __restrict__ out,
                                   const float* __restrict__ lse, float* __restrict__ delta,
                                   float* __restrict__ lse2, long T, int S, int Hq, int ld_out,
                                   int ld_dout, float4* __restrict__ acc4, long n_acc4) {
+  pdl_trigger();
+  pdl_wait();
   constexpr int TPH = D / 8;  // threads per (token, head)
   const long gid = static_cast<long>(blockIdx.x) * blockDim.x + threadIdx.x;
   {
@@ -599,6 +604,8 @@ __global__ void fa_bwd_post_kernel(const float* __restrict__ acc, __nv_bfloat16*
                                    float scale, const float* __restrict__ cos_t,
                                    const float* __restrict__ sin_t,
                                    const int* __restrict__ position_ids, int S) {
+  pdl_trigger();
+  pdl_wait();
   const int half = D / 2;
   const int vph = half / 8;                 // threads per head
   const int heads = ncols / D;
@@ -659,7 +666,7 @@ static int launch_fa_bwd(const CUtensorMap& tq, const CUtensorMap& tdo, const CU
     attr = true;
   }
   const int grid = (p.S / FAB_BLK) * p.batch * p.n_groups * (p.g / p.hpc);
-  fa_bwd_kernel<D, QS, NP, NDS, NST><<<grid, FAB_THREADS, L::TOTAL, st>>>(tq, tdo, tacc, p);
+  launch_pdl(fa_bwd_kernel<D, QS, NP, NDS, NST>, grid, FAB_THREADS, L::TOTAL, st, tq, tdo, tacc, p);
   return cudaGetLastError() == cudaSuccess ? 0 : -11;
 }
 
@@ -700,12 +707,12 @@ extern "C" int ft_attn_bwd(const void* dout, const void* qkv, const void* out, c
     const long threads = T * Hq * (D / 8);
     const int blocks = static_cast<int>((threads + 255) / 256);
     if (D == 64)
-      fa_bwd_pre_kernel<64><<<blocks, 256, 0, st>>>((const __nv_bfloat16*)out,
+      launch_pdl(fa_bwd_pre_kernel<64>, blocks, 256, 0, st, (const __nv_bfloat16*)out,
                                                     (const __nv_bfloat16*)dout, (const float*)lse,
                                                     d_delta, d_lse2, T, S, Hq, ld_out, ld_dout,
                                                     static_cast<float4*>(acc), n_acc4);
     else
-      fa_bwd_pre_kernel<128><<<blocks, 256, 0, st>>>((const __nv_bfloat16*)out,
+      launch_pdl(fa_bwd_pre_kernel<128>, blocks, 256, 0, st, (const __nv_bfloat16*)out,
                                                      (const __nv_bfloat16*)dout, (const float*)lse,
                                                      d_delta, d_lse2, T, S, Hq, ld_out, ld_dout,
                                                      static_cast<float4*>(acc), n_acc4);
@@ -748,7 +755,7 @@ extern "C" int ft_attn_bwd(const void* dout, const void* qkv, const void* out, c
     const long total = T * (ncols / 16);
     long blocks = (total + 255) / 256;
     if (blocks > 148 * 16) blocks = 148 * 16;
-    fa_bwd_post_kernel<<<static_cast<int>(blocks), 256, 0, st>>>(
+    launch_pdl(fa_bwd_post_kernel, static_cast<int>(blocks), 256, 0, st, 
         (const float*)acc, (__nv_bfloat16*)dqkv, T, ncols, ncols, ld_qkv, g, D, scale,
         (const float*)cos_t, (const float*)sin_t, (const int*)position_ids, S);
     if (cudaGetLastError() != cudaSuccess) return -7;

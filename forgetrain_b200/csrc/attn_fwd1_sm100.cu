@@ -17,6 +17,7 @@
 // issued behind the P V product that reads them (the tensor pipe runs one thread's products in
 // order), so a CTA alternates softmax and tensor work, and the OTHER resident CTA fills the gaps.
 // Shared memory: Q, one K and one V stage of 32 KB each.
+#include "launch.h"
 #include "ptx.cuh"
 #include "tma_host.h"
 
@@ -56,6 +57,7 @@ template <int D>
 __global__ void __launch_bounds__(FA1_THREADS, 2)
 fa_fwd1_kernel(const __grid_constant__ CUtensorMap tm_qkv, const __grid_constant__ CUtensorMap tm_out,
                const FaFwd1Params p) {
+  pdl_trigger();
   using L = FaFwd1Smem<D>;
   using C = FaFwd1Cfg<D>;
   constexpr int KS = C::STAGES, VS = C::STAGES, NBOX = D / 64;
@@ -118,6 +120,7 @@ fa_fwd1_kernel(const __grid_constant__ CUtensorMap tm_qkv, const __grid_constant
   tc_fence_before();
   __syncthreads();
   tc_fence_after();
+  pdl_wait();
   const uint32_t tmem_base = *tmem_slot;
   const uint32_t tmem_S = tmem_base;          // 128 columns
   const uint32_t tmem_O = tmem_base + 128;    // D
@@ -389,7 +392,7 @@ static int launch_fa_fwd1_t(const CUtensorMap& tq, const CUtensorMap& to, int S,
   p.lse = lse;
   p.status = status;
   const int grid = (S / FA1_BLK) * batch * Hq;
-  fa_fwd1_kernel<D><<<grid, FA1_THREADS, L::TOTAL, st>>>(tq, to, p);
+  launch_pdl(fa_fwd1_kernel<D>, grid, FA1_THREADS, L::TOTAL, st, tq, to, p);
   return cudaGetLastError() == cudaSuccess ? 0 : -11;
 }
 

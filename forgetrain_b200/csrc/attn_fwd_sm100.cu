@@ -23,6 +23,7 @@
 //
 // Replaces the reference's Hopper FlashAttention forward kernels
 // (ops/attention/flash_attn_dsl/flash_fwd.py:31-660, src/flash_attn_dsl/flash_fwd.py:1-803).
+#include "launch.h"
 #include "ptx.cuh"
 #include "tma_host.h"
 
@@ -76,6 +77,7 @@ template <int D, int KS, int VS>
 __global__ void __launch_bounds__(FA_THREADS, 1)
 fa_fwd_kernel(const __grid_constant__ CUtensorMap tm_qkv, const __grid_constant__ CUtensorMap tm_out,
               const FaFwdParams p) {
+  pdl_trigger();
   using L = FaFwdSmem<D, KS, VS>;
   extern __shared__ uint8_t smem_raw[];
   uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) &
@@ -137,6 +139,7 @@ fa_fwd_kernel(const __grid_constant__ CUtensorMap tm_qkv, const __grid_constant_
   tc_fence_before();
   __syncthreads();
   tc_fence_after();
+  pdl_wait();
   const uint32_t tmem_base = *tmem_slot;
   const uint32_t tmem_S[2] = {tmem_base, tmem_base + 128};
   const uint32_t tmem_O[2] = {tmem_base + 256, tmem_base + 256 + D};
@@ -453,7 +456,7 @@ static int launch_fa_fwd(const CUtensorMap& tq, const CUtensorMap& to, const FaF
     attr = true;
   }
   const int grid = (p.S / (2 * FA_BLK)) * p.batch * p.Hq;
-  fa_fwd_kernel<D, KS, VS><<<grid, FA_THREADS, L::TOTAL, st>>>(tq, to, p);
+  launch_pdl(fa_fwd_kernel<D, KS, VS>, grid, FA_THREADS, L::TOTAL, st, tq, to, p);
   return cudaGetLastError() == cudaSuccess ? 0 : -11;
 }
 

@@ -8,6 +8,7 @@
 // These replace the reference's Triton kernels
 // (exports/train_engine_0.5B/src/training_engine_tensor/triton_kernels.py:39-1397 and
 // exports/train_engine_8b/src/training_engine_tensor/kernels.py:144-2054).
+#include "launch.h"
 #include "ptx.cuh"
 #include "swiglu_math.cuh"
 
@@ -57,6 +58,8 @@ __global__ void embedding_fwd_kernel(const int64_t* __restrict__ ids,
                                      const __nv_bfloat16* __restrict__ w,
                                      __nv_bfloat16* __restrict__ out, int T, int H, float scale,
                                      int vocab_start, int vocab_rows) {
+  pdl_trigger();
+  pdl_wait();
   const int t = blockIdx.x;
   const long id = ids[t] - vocab_start;
   const bool live = id >= 0 && id < vocab_rows;
@@ -79,6 +82,8 @@ __global__ void embedding_fwd_kernel(const int64_t* __restrict__ ids,
 __global__ void embedding_bwd_kernel(const int64_t* __restrict__ ids,
                                      const __nv_bfloat16* __restrict__ dy, float* __restrict__ dw,
                                      int T, int H, float scale, int vocab_start, int vocab_rows) {
+  pdl_trigger();
+  pdl_wait();
   const int t = blockIdx.x;
   const long id = ids[t] - vocab_start;
   if (id < 0 || id >= vocab_rows) return;
@@ -105,6 +110,8 @@ add_rmsnorm_fwd_kernel(const __nv_bfloat16* __restrict__ res, const __nv_bfloat1
                        const __nv_bfloat16* __restrict__ w, __nv_bfloat16* __restrict__ h_out,
                        __nv_bfloat16* __restrict__ y, float* __restrict__ rstd_out, int T, int H,
                        float eps) {
+  pdl_trigger();
+  pdl_wait();
   __shared__ float red[4];
   constexpr int ROWS_PER_CTA = 128 / TPR;
   const int sub = threadIdx.x / TPR;
@@ -164,6 +171,8 @@ rmsnorm_bwd_kernel(const __nv_bfloat16* __restrict__ dy, const __nv_bfloat16* __
                    const __nv_bfloat16* __restrict__ w, const float* __restrict__ rstd_in,
                    const __nv_bfloat16* dres, __nv_bfloat16* dx_out,
                    float* __restrict__ dw_partial, int T, int H) {
+  pdl_trigger();
+  pdl_wait();
   __shared__ float red[4];
   extern __shared__ float dw_smem[];  // [H] when TPR == 32 (cross-warp fold), unused otherwise
   constexpr int ROWS_PER_CTA = 128 / TPR;
@@ -266,6 +275,8 @@ constexpr int COLSUM_GROUPS = 32;
 __global__ void __launch_bounds__(32 * COLSUM_GROUPS)
 colsum_partials_kernel(const float* __restrict__ partial, float* __restrict__ out, int P, int H,
                        int accumulate) {
+  pdl_trigger();
+  pdl_wait();
   __shared__ float red[COLSUM_GROUPS][33];
   const int cx = threadIdx.x & 31, px = threadIdx.x >> 5;
   const int c = blockIdx.x * 32 + cx;
@@ -297,6 +308,8 @@ __global__ void rope_kernel(__nv_bfloat16* __restrict__ qkv, const float* __rest
                             const float* __restrict__ sin_t,
                             const int* __restrict__ position_ids, long T, int S, int n_groups,
                             int g, int D, int ld, int inverse) {
+  pdl_trigger();
+  pdl_wait();
   const int half = D / 2;
   const int vec_per_head = half / 8;
   const int rot_heads = n_groups * (g + 1);
@@ -339,6 +352,8 @@ __global__ void rope_kernel(__nv_bfloat16* __restrict__ qkv, const float* __rest
 __global__ void swiglu_fwd_kernel(const __nv_bfloat16* __restrict__ y1,
                                   __nv_bfloat16* __restrict__ act, long T, int F, int ld_y1,
                                   int ld_act) {
+  pdl_trigger();
+  pdl_wait();
   const int vpr = F / 8;
   const long total = T * vpr;
   for (long idx = (long)blockIdx.x * blockDim.x + threadIdx.x; idx < total;
@@ -361,6 +376,8 @@ __global__ void swiglu_bwd_kernel(const __nv_bfloat16* __restrict__ dact,
                                   const __nv_bfloat16* __restrict__ y1,
                                   __nv_bfloat16* __restrict__ dy1, long T, int F, int ld_dact,
                                   int ld_y1) {
+  pdl_trigger();
+  pdl_wait();
   const int vpr = F / 8;
   const long total = T * vpr;
   for (long idx = (long)blockIdx.x * blockDim.x + threadIdx.x; idx < total;
@@ -401,6 +418,8 @@ cross_entropy_kernel(__nv_bfloat16* __restrict__ logits, const int64_t* __restri
                      const float* __restrict__ mask, const float* __restrict__ valid_ptr,
                      float* __restrict__ stats, float* __restrict__ row_loss, int T, int V,
                      long ld, int vocab_start, float loss_scale, int phase) {
+  pdl_trigger();
+  pdl_wait();
   __shared__ float sm[CE_THREADS / 32], ss[CE_THREADS / 32];
   __shared__ float bc[2];
   const int row = blockIdx.x;
@@ -487,6 +506,8 @@ cross_entropy_kernel(__nv_bfloat16* __restrict__ logits, const int64_t* __restri
 // gtarget[T]) compute the masked per-row loss.
 __global__ void ce_row_loss_kernel(const float* __restrict__ stats, const float* __restrict__ mask,
                                    float* __restrict__ row_loss, int T) {
+  pdl_trigger();
+  pdl_wait();
   const int i = blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= T) return;
   const float mk = mask ? mask[i] : 1.f;
@@ -497,6 +518,8 @@ __global__ void ce_row_loss_kernel(const float* __restrict__ stats, const float*
 __global__ void __launch_bounds__(1024)
 reduce_sum_kernel(const float* __restrict__ x, long n, const float* __restrict__ valid_ptr,
                   float scale, float* __restrict__ out, int accumulate) {
+  pdl_trigger();
+  pdl_wait();
   __shared__ float red[32];
   float s = 0.f;
   for (long i = threadIdx.x; i < n; i += blockDim.x) s += x[i];
@@ -525,6 +548,8 @@ adamw_kernel(float* __restrict__ p32, float* __restrict__ m, float* __restrict__
              const float* __restrict__ g, __nv_bfloat16* __restrict__ p_bf16, long n,
              const float* __restrict__ hyper, const long* __restrict__ seg_end,
              const float* __restrict__ seg_wd, const float* __restrict__ seg_lr_mult, int nseg) {
+  pdl_trigger();
+  pdl_wait();
   const float lr = hyper[0], b1 = hyper[1], b2 = hyper[2], eps = hyper[3];
   const float inv_bc1 = 1.f / hyper[4], inv_bc2 = 1.f / hyper[5], clip = hyper[6];
   const long nvec = n / 4;
@@ -569,6 +594,8 @@ adamw_kernel(float* __restrict__ p32, float* __restrict__ m, float* __restrict__
 // out[0] += sum(x^2) (fp32 atomics over per-CTA partials; callers zero out[0] first)
 __global__ void __launch_bounds__(256)
 sumsq_kernel(const float* __restrict__ x, long n, float* __restrict__ out) {
+  pdl_trigger();
+  pdl_wait();
   __shared__ float red[8];
   float s = 0.f;
   const long nvec = n / 4;
@@ -593,6 +620,8 @@ sumsq_kernel(const float* __restrict__ x, long n, float* __restrict__ out) {
 // clip[0] = min(1, max_norm / (sqrt(sumsq[0]) + 1e-6)); norm_out[0] = sqrt(sumsq[0])
 __global__ void clip_coef_kernel(const float* __restrict__ sumsq, float max_norm,
                                  float* __restrict__ hyper_clip, float* __restrict__ norm_out) {
+  pdl_trigger();
+  pdl_wait();
   const float nrm = sqrtf(sumsq[0]);
   norm_out[0] = nrm;
   hyper_clip[0] = max_norm > 0.f ? fminf(1.f, max_norm / (nrm + 1e-6f)) : 1.f;
@@ -606,6 +635,8 @@ __global__ void clip_coef_kernel(const float* __restrict__ sumsq, float max_norm
 // before the increment.
 __global__ void adam_hyper_kernel(int* __restrict__ step, const float* __restrict__ sched,
                                   float* __restrict__ hyper) {
+  pdl_trigger();
+  pdl_wait();
   const int it = step[0];
   const double max_lr = sched[0], min_lr = sched[1];
   const int warmup = (int)sched[2], decay = (int)sched[3], wsd = (int)sched[4];
@@ -648,7 +679,7 @@ extern "C" int ft_embedding_fwd(const void* ids, const void* w, void* out, int T
                                 float scale, int vocab_start, int vocab_rows,
                                 cudaStream_t st) {
   if (H % 8) return -1;
-  embedding_fwd_kernel<<<T, 128, 0, st>>>((const int64_t*)ids, (const __nv_bfloat16*)w,
+  launch_pdl(embedding_fwd_kernel, T, 128, 0, st, (const int64_t*)ids, (const __nv_bfloat16*)w,
                                           (__nv_bfloat16*)out, T, H, scale, vocab_start,
                                           vocab_rows);
   return FT_LAUNCH_OK();
@@ -658,7 +689,7 @@ extern "C" int ft_embedding_bwd(const void* ids, const void* dy, void* dw, int T
                                 float scale, int vocab_start, int vocab_rows,
                                 cudaStream_t st) {
   if (H % 8) return -1;
-  embedding_bwd_kernel<<<T, 128, 0, st>>>((const int64_t*)ids, (const __nv_bfloat16*)dy,
+  launch_pdl(embedding_bwd_kernel, T, 128, 0, st, (const int64_t*)ids, (const __nv_bfloat16*)dy,
                                           (float*)dw, T, H, scale, vocab_start, vocab_rows);
   return FT_LAUNCH_OK();
 }
@@ -685,7 +716,7 @@ extern "C" int ft_add_rmsnorm_fwd(const void* res, const void* x, const void* w,
   const int rows_per_cta = 128 / tpr;
   const int grid = grid_for((long)(T + rows_per_cta - 1) / rows_per_cta, 1, 16);
 #define CALL_FWD                                                                          \
-  add_rmsnorm_fwd_kernel<NV, TPR><<<grid, 128, 0, st>>>(                                  \
+  launch_pdl(add_rmsnorm_fwd_kernel<NV, TPR>, grid, 128, 0, st,                                   \
       (const __nv_bfloat16*)res, (const __nv_bfloat16*)x, (const __nv_bfloat16*)w,        \
       (__nv_bfloat16*)h_out, (__nv_bfloat16*)y, (float*)rstd, T, H, eps)
   FT_NORM_DISPATCH(1, 32, CALL_FWD)
@@ -714,7 +745,7 @@ extern "C" int ft_rmsnorm_bwd(const void* dy, const void* h, const void* w, cons
   const int grid = ft_rmsnorm_bwd_partials(T, H);
   const size_t smem = tpr == 32 ? (size_t)H * 4 : 0;
 #define CALL_BWD                                                                          \
-  rmsnorm_bwd_kernel<NV, TPR><<<grid, 128, smem, st>>>(                                   \
+  launch_pdl(rmsnorm_bwd_kernel<NV, TPR>, grid, 128, smem, st,                                    \
       (const __nv_bfloat16*)dy, (const __nv_bfloat16*)h, (const __nv_bfloat16*)w,         \
       (const float*)rstd, (const __nv_bfloat16*)dres, (__nv_bfloat16*)dx_out,             \
       (float*)dw_partial, T, H)
@@ -726,7 +757,7 @@ extern "C" int ft_rmsnorm_bwd(const void* dy, const void* h, const void* w, cons
   FT_NORM_DISPATCH(8, 128, CALL_BWD)
 #undef CALL_BWD
   if (cudaGetLastError() != cudaSuccess) return -100;
-  colsum_partials_kernel<<<(H + 31) / 32, 32 * COLSUM_GROUPS, 0, st>>>((const float*)dw_partial, (float*)dw,
+  launch_pdl(colsum_partials_kernel, (H + 31) / 32, 32 * COLSUM_GROUPS, 0, st, (const float*)dw_partial, (float*)dw,
                                                         grid, H, accumulate);
   return FT_LAUNCH_OK();
 }
@@ -736,7 +767,7 @@ extern "C" int ft_rope(void* qkv, const void* cos_t, const void* sin_t, const vo
                        cudaStream_t st) {
   if (D % 16 || ld % 8) return -1;
   const long total = T * n_groups * (g + 1) * (D / 16);
-  rope_kernel<<<grid_for(total, 256, 16), 256, 0, st>>>((__nv_bfloat16*)qkv, (const float*)cos_t,
+  launch_pdl(rope_kernel, grid_for(total, 256, 16), 256, 0, st, (__nv_bfloat16*)qkv, (const float*)cos_t,
                                                         (const float*)sin_t,
                                                         (const int*)position_ids, T, S, n_groups,
                                                         g, D, ld, inverse);
@@ -746,7 +777,7 @@ extern "C" int ft_rope(void* qkv, const void* cos_t, const void* sin_t, const vo
 extern "C" int ft_swiglu_fwd(const void* y1, void* act, long T, int F, int ld_y1, int ld_act,
                              cudaStream_t st) {
   if (F % 8 || ld_y1 % 8 || ld_act % 8) return -1;
-  swiglu_fwd_kernel<<<grid_for(T * (F / 8), 256, 16), 256, 0, st>>>(
+  launch_pdl(swiglu_fwd_kernel, grid_for(T * (F / 8), 256, 16), 256, 0, st, 
       (const __nv_bfloat16*)y1, (__nv_bfloat16*)act, T, F, ld_y1, ld_act);
   return FT_LAUNCH_OK();
 }
@@ -754,7 +785,7 @@ extern "C" int ft_swiglu_fwd(const void* y1, void* act, long T, int F, int ld_y1
 extern "C" int ft_swiglu_bwd(const void* dact, const void* y1, void* dy1, long T, int F,
                              int ld_dact, int ld_y1, cudaStream_t st) {
   if (F % 8 || ld_y1 % 8 || ld_dact % 8) return -1;
-  swiglu_bwd_kernel<<<grid_for(T * (F / 8), 256, 16), 256, 0, st>>>(
+  launch_pdl(swiglu_bwd_kernel, grid_for(T * (F / 8), 256, 16), 256, 0, st, 
       (const __nv_bfloat16*)dact, (const __nv_bfloat16*)y1, (__nv_bfloat16*)dy1, T, F, ld_dact,
       ld_y1);
   return FT_LAUNCH_OK();
@@ -767,7 +798,7 @@ extern "C" int ft_cross_entropy(void* logits, const void* labels, const void* ma
                                 long ld, int vocab_start, float loss_scale, int phase,
                                 cudaStream_t st) {
   if (ld % 8) return -1;
-  cross_entropy_kernel<<<T, CE_THREADS, 0, st>>>((__nv_bfloat16*)logits, (const int64_t*)labels,
+  launch_pdl(cross_entropy_kernel, T, CE_THREADS, 0, st, (__nv_bfloat16*)logits, (const int64_t*)labels,
                                                  (const float*)mask, (const float*)valid,
                                                  (float*)stats, (float*)row_loss, T, V, ld,
                                                  vocab_start, loss_scale, phase);
@@ -776,14 +807,14 @@ extern "C" int ft_cross_entropy(void* logits, const void* labels, const void* ma
 
 extern "C" int ft_ce_row_loss(const void* stats, const void* mask, void* row_loss, int T,
                               cudaStream_t st) {
-  ce_row_loss_kernel<<<(T + 255) / 256, 256, 0, st>>>((const float*)stats, (const float*)mask,
+  launch_pdl(ce_row_loss_kernel, (T + 255) / 256, 256, 0, st, (const float*)stats, (const float*)mask,
                                                       (float*)row_loss, T);
   return FT_LAUNCH_OK();
 }
 
 extern "C" int ft_reduce_sum(const void* x, long n, const void* valid, float scale, void* out,
                              int accumulate, cudaStream_t st) {
-  reduce_sum_kernel<<<1, 1024, 0, st>>>((const float*)x, n, (const float*)valid, scale,
+  launch_pdl(reduce_sum_kernel, 1, 1024, 0, st, (const float*)x, n, (const float*)valid, scale,
                                         (float*)out, accumulate);
   return FT_LAUNCH_OK();
 }
@@ -792,7 +823,7 @@ extern "C" int ft_adamw(void* p32, void* m, void* v, const void* g, void* p_bf16
                         const void* hyper, const void* seg_end, const void* seg_wd,
                         const void* seg_lr_mult, int nseg, cudaStream_t st) {
   if (n % 4) return -1;
-  adamw_kernel<<<grid_for(n / 4, 256, 16), 256, 0, st>>>(
+  launch_pdl(adamw_kernel, grid_for(n / 4, 256, 16), 256, 0, st, 
       (float*)p32, (float*)m, (float*)v, (const float*)g, (__nv_bfloat16*)p_bf16, n,
       (const float*)hyper, (const long*)seg_end, (const float*)seg_wd, (const float*)seg_lr_mult,
       nseg);
@@ -800,19 +831,19 @@ extern "C" int ft_adamw(void* p32, void* m, void* v, const void* g, void* p_bf16
 }
 
 extern "C" int ft_sumsq(const void* x, long n, void* out, cudaStream_t st) {
-  sumsq_kernel<<<grid_for(n / 4 + 1, 256, 8), 256, 0, st>>>((const float*)x, n, (float*)out);
+  launch_pdl(sumsq_kernel, grid_for(n / 4 + 1, 256, 8), 256, 0, st, (const float*)x, n, (float*)out);
   return FT_LAUNCH_OK();
 }
 
 extern "C" int ft_clip_coef(const void* sumsq, float max_norm, void* hyper_clip, void* norm_out,
                             cudaStream_t st) {
-  clip_coef_kernel<<<1, 1, 0, st>>>((const float*)sumsq, max_norm, (float*)hyper_clip,
+  launch_pdl(clip_coef_kernel, 1, 1, 0, st, (const float*)sumsq, max_norm, (float*)hyper_clip,
                                     (float*)norm_out);
   return FT_LAUNCH_OK();
 }
 
 extern "C" int ft_adam_hyper(void* step, const void* sched, void* hyper, cudaStream_t st) {
-  adam_hyper_kernel<<<1, 1, 0, st>>>((int*)step, (const float*)sched, (float*)hyper);
+  launch_pdl(adam_hyper_kernel, 1, 1, 0, st, (int*)step, (const float*)sched, (float*)hyper);
   return FT_LAUNCH_OK();
 }
 
@@ -852,7 +883,7 @@ extern "C" int ft_rmsnorm_bwd_noalloc(const void* dy, const void* h, const void*
   const int grid = want < 1 ? 1 : (want > FT_NOALLOC_MAX_PARTIALS ? FT_NOALLOC_MAX_PARTIALS : (int)want);
   const size_t smem = tpr == 32 ? (size_t)H * 4 : 0;
 #define CALL_BWD_NA                                                                       \
-  rmsnorm_bwd_kernel<NV, TPR><<<grid, 128, smem, st>>>(                                   \
+  launch_pdl(rmsnorm_bwd_kernel<NV, TPR>, grid, 128, smem, st,                                    \
       (const __nv_bfloat16*)dy, (const __nv_bfloat16*)h, (const __nv_bfloat16*)w,         \
       (const float*)rstd, (const __nv_bfloat16*)dres, (__nv_bfloat16*)dx_out, scratch, T, H)
   FT_NORM_DISPATCH(1, 32, CALL_BWD_NA)
@@ -863,6 +894,6 @@ extern "C" int ft_rmsnorm_bwd_noalloc(const void* dy, const void* h, const void*
   FT_NORM_DISPATCH(8, 128, CALL_BWD_NA)
 #undef CALL_BWD_NA
   if (cudaGetLastError() != cudaSuccess) return -100;
-  colsum_partials_kernel<<<(H + 31) / 32, 32 * COLSUM_GROUPS, 0, st>>>(scratch, (float*)dw, grid, H, accumulate);
+  launch_pdl(colsum_partials_kernel, (H + 31) / 32, 32 * COLSUM_GROUPS, 0, st, scratch, (float*)dw, grid, H, accumulate);
   return FT_LAUNCH_OK();
 }

@@ -21,6 +21,7 @@
 #include <string.h>
 #include <stdlib.h>
 
+#include "launch.h"
 #include "ptx.cuh"
 #include "swiglu_math.cuh"
 #include "tma_host.h"
@@ -342,6 +343,7 @@ __global__ void __launch_bounds__(GEMM_THREADS, 1)
 gemm_bf16_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUtensorMap tmB,
                  const __grid_constant__ CUtensorMap tmD, const __grid_constant__ CUtensorMap tmD2,
                  const GemmParams p) {
+  pdl_trigger();
   constexpr bool SWIGLU = EPI == EPI_SWIGLU_FWD;
   static_assert(EPI == EPI_PLAIN || BN == 256, "the fused SwiGLU epilogues are built for 256-column tiles");
   static_assert(MT == 1 || (MT == 2 && BN == 256 && EPI != EPI_SWIGLU_BWD),
@@ -387,6 +389,7 @@ gemm_bf16_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant_
   tc_fence_before();
   __syncthreads();
   tc_fence_after();
+  pdl_wait();
   const uint32_t tmem_base = *tmem_slot;
 
   const int total_tiles = p.total_units;
@@ -1002,8 +1005,7 @@ static int launch_gemm(const CUtensorMap& tmA, const CUtensorMap& tmB, const CUt
   const int total = p.total_units;
   int grid = total < max_ctas ? total : max_ctas;
   if (grid < 1) grid = 1;
-  gemm_bf16_kernel<BN, STAGES, EPI, MT>
-      <<<grid, GEMM_THREADS, L::TOTAL, stream>>>(tmA, tmB, tmD, tmD2, p);
+  launch_pdl(gemm_bf16_kernel<BN, STAGES, EPI, MT>, grid, GEMM_THREADS, L::TOTAL, stream, tmA, tmB, tmD, tmD2, p);
   return cudaGetLastError() == cudaSuccess ? 0 : -11;
 }
 

@@ -130,6 +130,17 @@ __device__ __forceinline__ bool mbar_wait_relaxed(uint64_t* bar, uint32_t parity
 }
 
 // ---------------------------------------------------------------------------------------
+// programmatic dependent launch (launch.h): let the next kernel of the stream start, and wait for
+// the previous one to have completed
+// ---------------------------------------------------------------------------------------
+__device__ __forceinline__ void pdl_trigger() {
+  asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+}
+__device__ __forceinline__ void pdl_wait() {
+  asm volatile("griddepcontrol.wait;" ::: "memory");
+}
+
+// ---------------------------------------------------------------------------------------
 // fences
 // ---------------------------------------------------------------------------------------
 __device__ __forceinline__ void fence_proxy_async_smem() {
