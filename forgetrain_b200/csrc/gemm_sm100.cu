@@ -40,9 +40,14 @@ constexpr int GEMM_PRODUCER_WARP2 = 10;
 constexpr int GEMM_EPI_WARPS = 8;    // two warps per TMEM lane quarter, each takes half the columns
 constexpr int GEMM_GROUP_M = 16;
 
+// EPI_CLUSTER: a unit's K range is accumulated in up to four pieces, which the epilogue adds up. The
+// tensor cores truncate as they add to an accumulator, so the error of a long chain grows with its
+// length: fp32 weight gradient 1280 x 1024 over 1024 tokens 9.9e-7 in one chain, 4.7e-7 in two.
+constexpr int CLUSTER_ACCS = 4;
+
 enum : int { OUT_BF16 = 0, OUT_F32 = 1, OUT_F32_ADD = 2 };
 // what the epilogue does besides scaling and storing the accumulator
-enum : int { EPI_PLAIN = 0, EPI_SWIGLU_FWD = 1, EPI_SWIGLU_BWD = 2 };
+enum : int { EPI_PLAIN = 0, EPI_SWIGLU_FWD = 1, EPI_SWIGLU_BWD = 2, EPI_CLUSTER = 3 };
 
 struct GemmParams {
   int M, N, K;
@@ -58,6 +63,8 @@ struct GemmParams {
   // last, partly filled wave is cut into two 128 x BN/2 halves (units 2i, 2i+1), so that the
   // tail of the schedule costs about 0.6 instead of 1.0 tile times. total_units counts both.
   int split_from, total_units;
+  void* d;            // EPI_CLUSTER: the output, written with plain stores
+  int ldd;
 };
 
 // MT: 128-row blocks of A per tile (1: 128 x BN tiles, 2: 256 x BN tiles)
@@ -304,6 +311,88 @@ __device__ __forceinline__ void drain_tile_swiglu_whole(const GemmParams& p,
   }
 }
 
+// EPI_CLUSTER: the reduction of one tile is split over the CTAs of a thread-block cluster. Each
+// leaves its fp32 partial in its own shared memory (the operand ring, which nothing uses any more),
+// in rows padded by 16 bytes: a warp whose lanes own rows then writes, and a warp that walks a row
+// reads, without bank conflicts. Then each CTA sums its share of the rows over all partials, in
+// rank order (the result does not depend on timing), and writes it out: no memset, no fp32
+// traffic to memory, and a bf16 result can be split too.
+template <int BN>
+__device__ __forceinline__ void stage_partial(uint32_t taddr, int kn, uint8_t* smem, int q,
+                                              int chalf, int lane) {
+  float* row = reinterpret_cast<float*>(smem) + (q * 32 + lane) * (BN + 4) + chalf * (BN / 2);
+  const int chunk = (kn + CLUSTER_ACCS - 1) / CLUSTER_ACCS;
+  const int naccs = (kn + chunk - 1) / chunk;
+#pragma unroll
+  for (int c = 0; c < BN / 64; ++c) {
+    float v[32];
+    uint32_t r[32];
+    tmem_ld32(taddr + chalf * (BN / 2) + c * 32, r);
+    tmem_ld_wait();
+#pragma unroll
+    for (int i = 0; i < 32; ++i) v[i] = __uint_as_float(r[i]);
+#pragma unroll 1
+    for (int k = 1; k < naccs; ++k) {
+      tmem_ld32(taddr + k * BN + chalf * (BN / 2) + c * 32, r);
+      tmem_ld_wait();
+#pragma unroll
+      for (int i = 0; i < 32; ++i) v[i] += __uint_as_float(r[i]);
+    }
+#pragma unroll
+    for (int i = 0; i < 8; ++i)
+      *reinterpret_cast<float4*>(row + c * 32 + 4 * i) =
+          make_float4(v[4 * i], v[4 * i + 1], v[4 * i + 2], v[4 * i + 3]);
+  }
+}
+
+template <int BN>
+__device__ __forceinline__ void sum_partials(const GemmParams& p, const uint8_t* smem, int row0,
+                                             int col0, int warp, int lane) {
+  static_assert(BN == 128, "a lane takes four columns of a row");
+  const int ncta = p.splitk;
+  const int per = (GEMM_BM + ncta - 1) / ncta;
+  const int first = static_cast<int>(cluster_ctarank()) * per;
+  const int last = min(first + per, GEMM_BM);
+  const int col = col0 + lane * 4;
+  for (int r = first + warp; r < last; r += GEMM_EPI_WARPS) {
+    const uint32_t at = smem_u32(smem) + (r * (BN + 4) + lane * 4) * 4;
+    float4 v[8];
+#pragma unroll
+    for (int c = 0; c < 8; ++c)
+      if (c < ncta) v[c] = ld_cluster_f4(mapa_u32(at, c));
+    float4 a = v[0];
+#pragma unroll
+    for (int c = 1; c < 8; ++c)
+      if (c < ncta) { a.x += v[c].x; a.y += v[c].y; a.z += v[c].z; a.w += v[c].w; }
+    a.x *= p.alpha; a.y *= p.alpha; a.z *= p.alpha; a.w *= p.alpha;
+    const int row = row0 + r;
+    if (row >= p.M || col >= p.N) continue;
+    const long off = static_cast<long>(row) * p.ldd + col;
+    if (p.out_mode == OUT_BF16) {
+      __nv_bfloat16* d = static_cast<__nv_bfloat16*>(p.d) + off;
+      if (col + 4 <= p.N) {
+        *reinterpret_cast<uint2*>(d) = make_uint2(pack_bf16x2(a.x, a.y), pack_bf16x2(a.z, a.w));
+      } else {
+        const float e[3] = {a.x, a.y, a.z};
+        for (int i = 0; i < p.N - col; ++i) d[i] = __float2bfloat16_rn(e[i]);
+      }
+    } else {
+      float* d = static_cast<float*>(p.d) + off;
+      if (col + 4 <= p.N) {
+        float4* d4 = reinterpret_cast<float4*>(d);
+        if (p.out_mode == OUT_F32_ADD) {
+          const float4 o = *d4;
+          a.x += o.x; a.y += o.y; a.z += o.z; a.w += o.w;
+        }
+        *d4 = a;
+      } else {
+        const float e[3] = {a.x, a.y, a.z};
+        for (int i = 0; i < p.N - col; ++i) d[i] = p.out_mode == OUT_F32_ADD ? d[i] + e[i] : e[i];
+      }
+    }
+  }
+}
+
 // Epilogue of the fused FC2 dgrad + SwiGLU backward kernel (EPI_SWIGLU_BWD), one warp's share.
 // The accumulator holds d act = alpha * dY W2 for 256 (or 128) columns of F; the warp owns 32 rows
 // and half of the columns and walks them in pieces of 32 columns. For every piece the gate box and
@@ -345,7 +434,8 @@ gemm_bf16_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant_
                  const GemmParams p) {
   pdl_trigger();
   constexpr bool SWIGLU = EPI == EPI_SWIGLU_FWD;
-  static_assert(EPI == EPI_PLAIN || BN == 256, "the fused SwiGLU epilogues are built for 256-column tiles");
+  static_assert(EPI == EPI_PLAIN || EPI == EPI_CLUSTER || BN == 256,
+                "the fused SwiGLU epilogues are built for 256-column tiles");
   static_assert(MT == 1 || (MT == 2 && BN == 256 && EPI != EPI_SWIGLU_BWD),
                 "two row blocks: 256-column tiles, and one staging buffer per epilogue warp");
   using L = GemmSmem<BN, STAGES, EPI == EPI_SWIGLU_BWD ? 2 : 1, MT>;
@@ -363,7 +453,8 @@ gemm_bf16_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant_
 
   const int warp = warp_idx_uniform();
   const int lane = threadIdx.x & 31;
-  constexpr uint32_t TMEM_COLS = 2 * BN;  // 256 or 512: two fp32 accumulators of BN columns
+  // two fp32 accumulators of BN columns; EPI_CLUSTER: CLUSTER_ACCS of them for one unit
+  constexpr uint32_t TMEM_COLS = (EPI == EPI_CLUSTER ? CLUSTER_ACCS : 2) * BN;
 
   if (threadIdx.x == 0) {
     for (int s = 0; s < STAGES; ++s) {
@@ -393,6 +484,11 @@ gemm_bf16_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant_
   const uint32_t tmem_base = *tmem_slot;
 
   const int total_tiles = p.total_units;
+  // EPI_CLUSTER: the p.splitk CTAs of a cluster take the K ranges of ONE tile, a unit each
+  const int unit0 = EPI == EPI_CLUSTER
+                        ? (blockIdx.x % p.splitk) * (p.m_tiles * p.n_tiles) + blockIdx.x / p.splitk
+                        : blockIdx.x;
+  const int ustep = EPI == EPI_CLUSTER ? total_tiles : gridDim.x;
 
   if (warp == 0 || warp == GEMM_PRODUCER_WARP2) {
     // ------------------------------ TMA producers ------------------------------
@@ -404,7 +500,7 @@ gemm_bf16_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant_
     if (lane < nA + nB) {
       int stage = 0;
       uint32_t phase = 0;
-      for (int tile = blockIdx.x; tile < total_tiles; tile += gridDim.x) {
+      for (int tile = unit0; tile < total_tiles; tile += ustep) {
         int mt, nt, kb, kn, half;
         decode_tile<MT>(p, tile, mt, nt, kb, kn, half);
         // a half tile loads only its half of the B boxes (MT == 1) or of the A boxes (MT == 2),
@@ -474,7 +570,7 @@ gemm_bf16_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant_
       int stage = 0;
       uint32_t phase = 0;
       int it = 0;
-      for (int tile = blockIdx.x; tile < total_tiles; tile += gridDim.x, ++it) {
+      for (int tile = unit0; tile < total_tiles; tile += ustep, ++it) {
         int mt, nt, kb, kn, half;
         decode_tile<MT>(p, tile, mt, nt, kb, kn, half);
         if constexpr (MT == 2) {
@@ -504,6 +600,29 @@ gemm_bf16_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant_
             if (++stage == STAGES) { stage = 0; phase ^= 1; }
           }
           it += blocks - 1;   // the loop header counts the other one
+          continue;
+        }
+        if constexpr (EPI == EPI_CLUSTER) {
+          const int chunk = (kn + CLUSTER_ACCS - 1) / CLUSTER_ACCS;
+          uint32_t tmem_d = tmem_base;
+          for (int ki = 0, in = 0; ki < kn; ++ki) {
+            mbar_wait(&full_bar[stage], phase, abort_flag, p.status, FT_ERR_WAIT_FULL);
+            tc_fence_after();
+            if (elect_one_sync()) {
+              const uint32_t sA = smem_base + stage * L::STAGE_BYTES;
+              const uint32_t a_lo = smem_desc_lo(sA, a_lbo);
+              const uint32_t b_lo = smem_desc_lo(sA + L::A_BYTES, b_lbo);
+              umma_ss_lo_dyn(tmem_d, a_lo, b_lo, idesc_full, in > 0 ? 1u : 0u);
+#pragma unroll
+              for (int kk = 1; kk < GEMM_BK / 16; ++kk)
+                umma_ss_lo<1>(tmem_d, a_lo + kk * a_kstep, b_lo + kk * b_kstep, idesc_full);
+              umma_commit(&empty_bar[stage]);
+              if (ki == kn - 1) umma_commit(&tfull_bar[0]);
+            }
+            __syncwarp();
+            if (++in == chunk) { in = 0; tmem_d += BN; }
+            if (++stage == STAGES) { stage = 0; phase ^= 1; }
+          }
           continue;
         }
         const uint32_t idesc = half < 0 ? idesc_full : idesc_half;
@@ -661,7 +780,7 @@ gemm_bf16_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant_
         if (lane == 0) mbar_arrive(&tempty_bar[buf]);
       }
     } else {
-    for (int tile = blockIdx.x; tile < total_tiles; tile += gridDim.x) {
+    for (int tile = unit0; tile < total_tiles; tile += ustep) {
       int mt, nt, kb, kn, half;
       decode_tile<MT>(p, tile, mt, nt, kb, kn, half);
       const int blocks = MT == 2 && half < 0 ? 2 : 1;
@@ -678,7 +797,9 @@ gemm_bf16_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant_
           __syncwarp();
           if (lane == 0) mbar_arrive(&tempty_bar[buf]);
         };
-        if (SWIGLU && MT == 2)
+        if constexpr (EPI == EPI_CLUSTER)
+          stage_partial<BN>(taddr, kn, smem, q, chalf, lane);
+        else if (SWIGLU && MT == 2)
           drain_tile_swiglu_whole(p, &tmD, &tmD2, taddr, row0, nt * 128, my_epi, lane, nstores,
                                   release);
         else if (SWIGLU)
@@ -701,6 +822,15 @@ gemm_bf16_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant_
   if (warp == 1) {
     tc_fence_after();
     tmem_dealloc(tmem_base, TMEM_COLS);
+  }
+  if constexpr (EPI == EPI_CLUSTER) {
+    cluster_sync_all();   // every CTA's partial tile is in its shared memory
+    if (warp >= 2 && warp < 2 + GEMM_EPI_WARPS && unit0 < total_tiles) {
+      int mt, nt, kb, kn, half;
+      decode_tile<MT>(p, unit0, mt, nt, kb, kn, half);
+      sum_partials<BN>(p, smem, mt * GEMM_BM, nt * BN, warp - 2, lane);
+    }
+    cluster_sync_all();   // nobody leaves while another CTA still reads its partial
   }
 }
 
@@ -1003,9 +1133,10 @@ static int launch_gemm(const CUtensorMap& tmA, const CUtensorMap& tmB, const CUt
     attr_set = true;
   }
   const int total = p.total_units;
-  int grid = total < max_ctas ? total : max_ctas;
+  int grid = total < max_ctas || EPI == EPI_CLUSTER ? total : max_ctas;
   if (grid < 1) grid = 1;
-  launch_pdl(gemm_bf16_kernel<BN, STAGES, EPI, MT>, grid, GEMM_THREADS, L::TOTAL, stream, tmA, tmB, tmD, tmD2, p);
+  launch_pdl_cluster(gemm_bf16_kernel<BN, STAGES, EPI, MT>, EPI == EPI_CLUSTER ? p.splitk : 1, grid,
+                     GEMM_THREADS, L::TOTAL, stream, tmA, tmB, tmD, tmD2, p);
   return cudaGetLastError() == cudaSuccess ? 0 : -11;
 }
 
@@ -1032,41 +1163,101 @@ static int auto_splitk(int tiles, int k_iters, int max_ctas) {
 }
 
 struct GemmPlan {
-  int mt, splitk;
+  int mt, bn, splitk, cluster;
 };
 
-// Tile height and split of the reduction for 256-column tiles, by the estimated length of the
-// schedule. Unit: a hundredth of what one k-step of a 128 x 256 tile costs a CTA (about 400 ns under
-// load). Measured over T = 256 .. 16384 tokens with the shapes of the 0.5B and 8B layers, operands
-// rotated through more than L2, back to back in a graph (us, 128 x 256 -> 256 x 256 tiles):
-//   fc1 fwd   16384 x 8192 x 1024   214 -> 197      fc1 wgrad  8192 x 1024 x 16384  211 -> 185
-//   fc2 fwd   16384 x 1024 x 4096   104 -> 99       8B qkv fwd  4096 x 4608 x 4096  111 -> 101
-//   8B fc2 fwd 4096 x 4096 x 16384  414 -> 368      8B wo wgrad 8192 x 4096 x 4096  215 -> 194
-//   wo fwd    16384 x 1024 x 1024   31.0 -> 31.2    qkv fwd    16384 x 1280 x 1024  37.9 -> 40.0
-//   fc2 fwd    4096 x 1024 x 4096   30.9 -> 38.4    8B qkv fwd  1024 x 4608 x 4096  30.8 -> 37.5
-// The last four are short of tiles: a 256 x 256 tile costs 1.75 of a 128 x 256 one, a half of it 1.2
-// (a half of the small one 0.8), and its epilogue is exposed for about 2.5 (fp32: 4) k-steps. A
-// split costs the memset and the reduce-adds, about 16 k-steps (10 without the memset): QKV wgrad
-// at 1024 tokens 13.1 us split in two, 10.2 whole.
-static GemmPlan pick_plan(int M, int N, int k_iters, bool f32, int accumulate, int max_ctas) {
-  GemmPlan best{1, 1};
+// How many clusters of `size` CTAs of the split-reduction kernel the device holds at once (a cluster
+// lies inside one GPC: 32 of four CTAs fit a B200, but fewer than 16 of seven or eight).
+static int max_clusters(int size) {
+  static int known[9] = {0};
+  if (known[size] == 0) {
+    using L = GemmSmem<128, 6>;
+    cudaLaunchAttribute attr;
+    attr.id = cudaLaunchAttributeClusterDimension;
+    attr.val.clusterDim.x = size;
+    attr.val.clusterDim.y = attr.val.clusterDim.z = 1;
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3(size);
+    cfg.blockDim = dim3(GEMM_THREADS);
+    cfg.dynamicSmemBytes = L::TOTAL;
+    cfg.attrs = &attr;
+    cfg.numAttrs = 1;
+    int n = 0;
+    auto kernel = gemm_bf16_kernel<128, 6, EPI_CLUSTER>;
+    if (cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, L::TOTAL) !=
+            cudaSuccess ||
+        cudaOccupancyMaxActiveClusters(&n, kernel, &cfg) != cudaSuccess) {
+      cudaGetLastError();   // no clusters of this size here: the rule does not use them
+      n = 0;
+    }
+    known[size] = n > 0 ? n : -1;
+  }
+  return known[size];
+}
+
+// Tile shape and split of the reduction, by the estimated length of the schedule. Unit: a hundredth
+// of what one k-step of a 128 x 256 tile costs a CTA (about 390 ns with every SM loading: an SM takes
+// in about 66 bytes per cycle whatever the tile). Measured over T = 256 .. 16384 tokens with the shapes
+// of the 0.5B and 8B layers, operands rotated through more than L2, back to back in a graph (us):
+//   128 x 256 -> 256 x 256 tiles
+//     fc1 fwd   16384 x 8192 x 1024   214 -> 197      fc1 wgrad  8192 x 1024 x 16384  211 -> 185
+//     fc2 fwd   16384 x 1024 x 4096   104 -> 99       8B qkv fwd  4096 x 4608 x 4096  111 -> 101
+//     8B fc2 fwd 4096 x 4096 x 16384  414 -> 368      8B wo wgrad 8192 x 4096 x 4096  215 -> 194
+//     wo fwd    16384 x 1024 x 1024   31.0 -> 31.2    qkv fwd    16384 x 1280 x 1024  37.9 -> 40.0
+//     fc2 fwd    4096 x 1024 x 4096   30.9 -> 38.4    8B qkv fwd  1024 x 4608 x 4096  30.8 -> 37.5
+//   The last four are short of tiles: a 256 x 256 tile costs 1.75 of a 128 x 256 one, a half of it 1.2
+//   (a half of the small one 0.8), and its epilogue is exposed for about 2.5 (fp32: 4) k-steps.
+//   128 x 256 cut in halves -> 128 x 128 tiles (0.66) -> their reduction split in a cluster of S CTAs
+//     fc1 dgrad   256 x 1024 x 8192   40.0 -> 31.3 -> 12.4 (S = 6)     fc2 fwd  512 x 1024 x 4096  22.7 -> 18.0
+//     fc1 dgrad   512 x 1024 x 8192   39.8 -> 32.1 -> 15.1 (S = 4)     fc2 fwd 2048 x 1024 x 4096  23.4 -> 20.1
+//     fc1 dgrad  1024 x 1024 x 8192   40.6 -> 33.0 -> 23.4 (S = 2)     qkv fwd 1536 x 1280 x 1024   8.7 ->  8.1
+//     fc1 dgrad  2048 x 1024 x 8192   40.8 -> 36.2                     8B fc1 dgrad 256 x 4096 x 32768  156 -> 118 -> 73
+//     wo dgrad    256 x 1024 x 1024    7.0 ->  6.9 ->  6.8 (S = 4)
+//   A cluster costs its launch, two barriers and the exchange: 3.5 us, 9 k-steps.
+//   fp32 results: splitting over the grid costs the memset and the reduce-adds, 16.5 k-steps, or 7
+//   into a gradient that is accumulated anyway (wo wgrad 1024 x 1024 x T, T = 2048: 128 x 128 12.4,
+//   cluster of two 11.5, grid split in four 13.2; accumulating 12.6, 13.2, 10.4).
+// Exactness: the forward pass (kind 0) is never split, so that all tile shapes give the same bits and a
+// token's result does not depend on how many tokens are in the batch. A weight gradient (kind 2; 1:
+// data gradient) is summed in at least as many pieces as its tokens are split into with 128 x 256
+// tiles: error against 64 bits, 1280 x 1024 over 1024 tokens, 4.7e-7 -> 2.3e-7.
+static GemmPlan pick_plan(int M, int N, int k_iters, int kind, int accumulate, int max_ctas) {
+  GemmPlan best{1, 256, 1, 1};
   long best_cost = 0;
+  const bool f32 = kind == 2;
+  auto offer = [&](const GemmPlan& plan, long cost) {
+    if (best_cost == 0 || cost < best_cost) {
+      best_cost = cost;
+      best = plan;
+    }
+  };
+  int chains = 1;   // pieces in which an fp32 result's reduction is summed at least
+  const long mt128 = (M + GEMM_BM - 1) / GEMM_BM;
   for (int mt = 1; mt <= 2; ++mt) {
-    const long tiles = static_cast<long>((M + GEMM_BM * mt - 1) / (GEMM_BM * mt)) * ((N + 255) / 256);
+    const long tiles = (mt128 + mt - 1) / mt * ((N + 255) / 256);
     const int max_split = f32 && tiles < max_ctas ? auto_splitk(static_cast<int>(tiles), k_iters, max_ctas) : 1;
-    for (int s = 1; s <= max_split; ++s) {
+    if (mt == 1) chains = max_split;
+    for (int s = mt == 1 ? max_split : chains < max_split ? chains : max_split; s <= max_split; ++s) {
       const long units = tiles * s, waves = units / max_ctas, rem = units % max_ctas;
       const long k = (k_iters + s - 1) / s;
       const long whole = mt == 2 ? 175 * k + (f32 ? 400 : 250) : 100 * k;
       const long half = mt == 2 ? 120 * k + 250 : 80 * k;
       long cost = waves * whole;
       if (rem) cost += s == 1 && 2 * rem <= max_ctas ? half : whole;
-      if (s > 1) cost += accumulate ? 1000 : 1650;
+      if (s > 1) cost += accumulate ? 700 : 1650;
       if (mt == 2) cost += cost / 50;   // a tie stays with the smaller tile
-      if (best_cost == 0 || cost < best_cost) {
-        best_cost = cost;
-        best = GemmPlan{mt, s};
-      }
+      offer(GemmPlan{mt, 256, s, 1}, cost);
+    }
+  }
+  const long tiles = mt128 * ((N + 127) / 128);
+  if (tiles <= max_ctas) {   // with more tiles the wider ones load less per product
+    // fp32: through the cluster kernel, with its four accumulators, also without a cluster
+    if (!f32 || chains <= CLUSTER_ACCS) offer(GemmPlan{1, 128, 1, f32 ? -1 : 1}, 66L * k_iters);
+    for (int c = 2; kind > 0 && c <= 8 && tiles * c <= max_ctas && 2 * c <= k_iters; ++c) {
+      const long cost = 66L * ((k_iters + c - 1) / c) + 900;
+      // asked only where it could win: the occupancy query runs once per cluster size
+      if (cost < best_cost && (!f32 || chains <= CLUSTER_ACCS * c) && tiles <= max_clusters(c))
+        offer(GemmPlan{1, 128, 1, c}, cost);
     }
   }
   return best;
@@ -1117,33 +1308,37 @@ static int launch_gemm_pair(const CUtensorMap& tmA, const CUtensorMap& tmB,
 //   a_mn == 0: A is stored [M][lda] (reduction index contiguous); a_mn == 1: A is stored
 //   [K][lda] (row index contiguous). Same for B with N. out_dtype: 0 bf16, 1 fp32.
 //   accumulate != 0 (fp32 only): D += result. splitk <= 0 picks a split automatically
-//   (fp32 only); bn in {0 (auto), 128, 256: one 128 x bn tile, 512: a 256 x 256 tile per CTA}. All leading dimensions in elements; every base
+//   (fp32 only); bn in {0 (auto), 128, 256: one 128 x bn tile, 512: a 256 x 256 tile per CTA,
+//   1000 + S: 128 x 128 tiles whose reduction is split inside clusters of S = 2 .. 8 CTAs}. All leading dimensions in elements; every base
 //   pointer 16-byte aligned and every leading dimension a multiple of 8 (bf16) / 4 (fp32).
 extern "C" int ft_gemm_bf16(const void* A, const void* B, void* D, int M, int N, int K, int lda,
                             int ldb, int ldd, int a_mn, int b_mn, int out_dtype, int accumulate,
                             float alpha, int splitk, int bn, int max_ctas, int* status,
                             cudaStream_t stream) {
   using namespace ft;
+  const int cluster = bn > 1000 && bn <= 1008 ? bn - 1000 : 0;
   if (M <= 0 || N <= 0 || K <= 0) return -1;
   if (out_dtype == 0 && accumulate) return -2;
   const int sms = num_sms();
   if (max_ctas <= 0 || max_ctas > sms) max_ctas = sms;
   const int k_iters = (K + GEMM_BK - 1) / GEMM_BK;
-  if (out_dtype == 0) splitk = 1;
-  int mt = bn == 512 ? 2 : 1;
-  const bool pick = bn != 128 && bn != 256 && bn != 512 && N > 128 && (out_dtype == 0 || splitk <= 0);
-  if (bn == 512) bn = 256;
+  GemmPlan plan{bn == 512 ? 2 : 1, bn, splitk, 1};
+  if (out_dtype == 0) splitk = plan.splitk = 1;
+  const bool given = bn == 128 || bn == 256 || bn == 512;
   if (bn != 128 && bn != 256) bn = (N <= 128) ? 128 : 256;
-  if (pick) {
-    const GemmPlan plan = pick_plan(M, N, k_iters, out_dtype == 1, accumulate, max_ctas);
-    mt = plan.mt;
-    splitk = plan.splitk;
-  }
+  plan.bn = bn;
+  if (cluster > 0) plan = GemmPlan{1, 128, 1, cluster == 1 ? -1 : cluster < k_iters ? cluster : k_iters};
+  else if (!given && N > 128 && (out_dtype == 0 || splitk <= 0))
+    plan = pick_plan(M, N, k_iters, out_dtype == 1 ? 2 : b_mn ? 1 : 0, accumulate, max_ctas);
+  bn = plan.bn;
+  const int mt = plan.mt;
   const int m_tiles = (M + GEMM_BM * mt - 1) / (GEMM_BM * mt);
   const int n_tiles = (N + bn - 1) / bn;
+  splitk = plan.cluster > 1 ? plan.cluster : plan.cluster < 0 ? 1 : plan.splitk;
   if (splitk <= 0) splitk = auto_splitk(m_tiles * n_tiles, k_iters, max_ctas);
   if (splitk > k_iters) splitk = k_iters;
   if (splitk < 1) splitk = 1;
+  const bool in_cluster = plan.cluster != 1;
 
   GemmParams p;
   p.M = M; p.N = N; p.K = K;
@@ -1156,8 +1351,10 @@ extern "C" int ft_gemm_bf16(const void* A, const void* B, void* D, int M, int N,
   p.split_from = p.total_units = m_tiles * n_tiles * splitk;
   if (bn == 256 && splitk == 1) cut_tail(p, max_ctas);
   if (out_dtype == 0) p.out_mode = OUT_BF16;
-  else p.out_mode = (accumulate || splitk > 1) ? OUT_F32_ADD : OUT_F32;
-  if (out_dtype == 1 && !accumulate && splitk > 1) {
+  else p.out_mode = (accumulate || (splitk > 1 && !in_cluster)) ? OUT_F32_ADD : OUT_F32;
+  p.d = D;
+  p.ldd = ldd;
+  if (out_dtype == 1 && !accumulate && splitk > 1 && !in_cluster) {
     if (cudaMemset2DAsync(D, static_cast<size_t>(ldd) * 4, 0, static_cast<size_t>(N) * 4, M,
                           stream) != cudaSuccess)
       return -3;
@@ -1175,6 +1372,8 @@ extern "C" int ft_gemm_bf16(const void* A, const void* B, void* D, int M, int N,
   else                rc = get_tmap_2d(&tmD, D, 4, M, N, ldd, 32, 32);
   if (rc) return -6;
 
+  if (in_cluster)
+    return launch_gemm<128, 6, EPI_CLUSTER>(tmA, tmB, tmD, tmD, p, max_ctas, stream);
   if (mt == 2) return launch_gemm<256, 3, EPI_PLAIN, 2>(tmA, tmB, tmD, tmD, p, max_ctas, stream);
   if (bn == 256) return launch_gemm<256, 4>(tmA, tmB, tmD, tmD, p, max_ctas, stream);
   return launch_gemm<128, 6>(tmA, tmB, tmD, tmD, p, max_ctas, stream);
@@ -1196,7 +1395,7 @@ extern "C" int ft_gemm_swiglu_bf16(const void* A, const void* W, void* Y, void* 
   // us. At K = 1024 a tile's main loop is shorter than the three stores and the activation of its
   // 256 x 128 outputs take the four warps of an accumulator: 253 -> 263 us at 16384 tokens.
   const int k_iters = (K + GEMM_BK - 1) / GEMM_BK;
-  const int mt = k_iters >= 32 && pick_plan(M, 2 * F, k_iters, false, 0, max_ctas).mt == 2 ? 2 : 1;
+  const int mt = k_iters >= 32 && pick_plan(M, 2 * F, k_iters, 0, 0, max_ctas).mt == 2 ? 2 : 1;
   GemmParams p;
   p.M = M; p.N = 2 * F; p.K = K;
   p.a_mn = 0; p.b_mn = 0;

@@ -17,19 +17,29 @@
 namespace ft {
 
 template <class... P, class... A>
-inline cudaError_t launch_pdl(void (*kernel)(P...), int grid, int block, size_t smem,
-                              cudaStream_t st, const A&... args) {
-  cudaLaunchAttribute attr;
-  attr.id = cudaLaunchAttributeProgrammaticStreamSerialization;
-  attr.val.programmaticStreamSerializationAllowed = 1;
+inline cudaError_t launch_pdl_cluster(void (*kernel)(P...), int cluster, int grid, int block,
+                                      size_t smem, cudaStream_t st, const A&... args) {
+  cudaLaunchAttribute attr[2];
+  attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  attr[0].val.programmaticStreamSerializationAllowed = 1;
+  attr[1].id = cudaLaunchAttributeClusterDimension;
+  attr[1].val.clusterDim.x = cluster;
+  attr[1].val.clusterDim.y = 1;
+  attr[1].val.clusterDim.z = 1;
   cudaLaunchConfig_t cfg = {};
   cfg.gridDim = dim3(grid);
   cfg.blockDim = dim3(block);
   cfg.dynamicSmemBytes = smem;
   cfg.stream = st;
-  cfg.attrs = &attr;
-  cfg.numAttrs = 1;
+  cfg.attrs = attr;
+  cfg.numAttrs = cluster > 1 ? 2 : 1;
   return cudaLaunchKernelEx(&cfg, kernel, static_cast<P>(args)...);
+}
+
+template <class... P, class... A>
+inline cudaError_t launch_pdl(void (*kernel)(P...), int grid, int block, size_t smem,
+                              cudaStream_t st, const A&... args) {
+  return launch_pdl_cluster(kernel, 1, grid, block, smem, st, args...);
 }
 
 }  // namespace ft
