@@ -25,7 +25,12 @@ import torch
 from .. import ops
 from ..config import ModelSpec
 from ..parallel.tp import NO_TP, TPContext
+from ..ops.layer import Block, BlockSaved
 from .params import ParamStore, vocab_shard_rows
+
+
+def _flat_positions(position_ids):
+    return None if position_ids is None else position_ids.reshape(-1).to(torch.int32)
 
 
 class LayerSaved:
@@ -71,7 +76,7 @@ class MiniCPM4:
             self.local_groups, self.local_g = 1, spec.heads_per_group // rep
         self.vocab_rows = vocab_shard_rows(spec.vocab_size, tpn) if tpn > 1 else spec.vocab_size
         self.vocab_start = tp.rank * self.vocab_rows if tpn > 1 else 0
-        self._saved: list[LayerSaved] = []
+        self._saved: list[LayerSaved | BlockSaved] = []
         self._head_saved = None
         # set to a dict to have the backward record a few intermediate gradients in it
         self.diagnostics: dict | None = None
@@ -87,7 +92,20 @@ class MiniCPM4:
         self._wgrad_done: dict[str, object] = {}
         # FC1 + SwiGLU in one kernel where FC1 is a plain local GEMM (no tensor parallelism)
         self.fuse_fc1_swiglu = tpn == 1 and os.environ.get("FT_FUSE_FC1_SWIGLU", "1") != "0"
+        # whole blocks in one native call where every op of them runs on this rank alone
+        self._block = None
+        if self.fuse_fc1_swiglu and dev.type == "cuda" and store.dtype == torch.bfloat16:
+            self._block = Block(spec, self.local_g, self.local_groups)
         self._ensure_rope(S)
+
+    def _block_takes(self, tensors, batch: int, position_ids) -> bool:
+        b, x = self._block, tensors[0]
+        if b is None or x.shape[0] % batch:
+            return False
+        S = x.shape[0] // batch
+        return (all(t is None or (b.takes(t, S) and t.shape == x.shape) for t in tensors)
+                and S <= self.cos.shape[0]
+                and (position_ids is None or (position_ids.is_cuda and position_ids.numel() == x.shape[0])))
 
     def _ensure_rope(self, S: int) -> None:
         if self.cos.shape[0] < S:
@@ -111,11 +129,18 @@ class MiniCPM4:
         sp, p, tp = self.spec, self.p, self.tp
         if self.param_gate is not None:
             self.param_gate(prefix)
+        x_in = h_prev if h_prev is not None else branch
+        res = branch if h_prev is not None else None
+        if self._block_takes((x_in, res), batch, position_ids):
+            w = [p[f"{prefix}.{n}"] for n in (
+                "attention_norm.weight", "attention.wqkv.weight", "attention.wo.weight", "ffn_norm.weight",
+                "feed_forward.wfc1.weight", "feed_forward.w2.weight")]
+            return self._block.forward(w, res, x_in, self.cos, self.sin, _flat_positions(position_ids),
+                                       x_in.shape[0] // batch, not self.recompute_attn, not self.recompute_mlp)
         r = sp.mup_residual_scale
         sv = LayerSaved()
-        x_in = h_prev if h_prev is not None else branch
         h_in, n1, sv.rs1 = ops.add_rmsnorm_fwd(
-            branch if h_prev is not None else None, x_in, p[f"{prefix}.attention_norm.weight"],
+            res, x_in, p[f"{prefix}.attention_norm.weight"],
             sp.norm_epsilon, tp.gather_dest(f"{prefix}.n1", x_in.shape[0], x_in.shape[1]))
         sv.h_in = h_in
         qkv, sv.n1_full = tp.linear_gather(n1, p[f"{prefix}.attention.wqkv.weight"],
@@ -262,6 +287,18 @@ class MiniCPM4:
         # gradients of the LAST block are what a numerical comparison with another engine looks
         # at first (reference backward.py:211-252: the ``diagnostics`` dict)
         diag = self.diagnostics if prefix == f"layers.{sp.num_layers - 1}" else None
+        if isinstance(sv, BlockSaved):
+            if diag is None and self._block_takes((dh,), batch, position_ids):
+                b, side = self._block, self.wgrad_stream
+                b.backward_ffn(sv, dh, (p[n_w2], p[n_fc1], p[n_fn]), (g[n_w2], g[n_fc1], g[n_fn]), accumulate, side)
+                for name in (n_w2, n_fc1, n_fn):
+                    emit(name)
+                b.backward_attn(sv, dh, (p[n_wo], p[n_qkv], p[n_an]), (g[n_wo], g[n_qkv], g[n_an]), self.cos,
+                                self.sin, _flat_positions(position_ids), dh.shape[0] // batch, accumulate, side)
+                for name in (n_qkv, n_an, n_wo):
+                    emit(name)
+                return dh
+            sv = self._block.unpack(sv, LayerSaved(), dh.shape[0] // batch)
         if diag is not None:
             diag["d_hidden_into_last_layer"] = dh.detach().clone()
         # ---- feed-forward branch

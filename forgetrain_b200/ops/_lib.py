@@ -51,7 +51,7 @@ def lib():
 
 # kernels launched per entry point (entry points not listed launch one kernel)
 _KERNELS_PER_CALL = {"ft_rmsnorm_bwd": 2, "ft_attn_bwd": 3, "ft_rmsnorm_bwd_partials": 0,
-                     "ft_tmap_cache_clear": 0}
+                     "ft_tmap_cache_clear": 0, "ft_layer_fwd": 8, "ft_layer_bwd_ffn": 6, "ft_layer_bwd_attn": 9}
 _LAUNCHES = [0]
 
 
@@ -99,7 +99,8 @@ def ptr(t: torch.Tensor | None) -> c_void_p:
 
 
 def stream() -> c_void_p:
-    return c_void_p(torch.cuda.current_stream().cuda_stream)
+    # the handle itself: building the Stream object around it takes longer than a launch
+    return c_void_p(torch._C._cuda_getCurrentRawStream(torch._C._cuda_getDevice()))
 
 
 _STATUS: dict[int, torch.Tensor] = {}
@@ -116,7 +117,8 @@ STATUS_MESSAGES = {
 
 def status_word(device: torch.device | int | None = None) -> torch.Tensor:
     """Per-device int32 word that kernels set when one of their bounded waits gives up."""
-    dev = torch.cuda.current_device() if device is None else torch.device(device).index
+    dev = device.index if isinstance(device, torch.device) else \
+        (None if device is None else torch.device(device).index)
     if dev is None:
         dev = torch.cuda.current_device()
     t = _STATUS.get(dev)

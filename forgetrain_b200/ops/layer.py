@@ -105,7 +105,7 @@ class Block:
         n = math.prod(shape) * dtype.itemsize
         return sv.keep[sv.offs[i]:sv.offs[i] + n].view(dtype).view(shape)
 
-    def unpack(self, sv: BlockSaved, into):
+    def unpack(self, sv: BlockSaved, into, seq: int):
         """The same as separate tensors, in the attributes of ``into`` (the op-by-op sequence's record)."""
         T, bf, f32 = sv.T, torch.bfloat16, torch.float32
         into.h_in = sv.h_in if sv.h_in is not None else self.piece(sv, 0, bf, T, self.H)
@@ -113,6 +113,9 @@ class Block:
         into.n2_full = self.piece(sv, 3, bf, T, self.H)
         into.rs1, into.rs2 = self.piece(sv, 4, f32, T), self.piece(sv, 5, f32, T)
         into.h_mid, into.attn, into.y1, into.act = sv.h_mid, sv.attn, sv.y1, sv.act
+        if sv.attn is not None:
+            B = T // seq
+            into.lse = self.piece(sv, 6, f32, B, self.G * self.g, seq)
         return into
 
     def backward_ffn(self, sv: BlockSaved, dh, w, g, accumulate: bool, side) -> None:
