@@ -364,10 +364,7 @@ __global__ void swiglu_fwd_kernel(const __nv_bfloat16* __restrict__ y1,
     unpack8(*reinterpret_cast<const bf16x8*>(y1 + t * ld_y1 + v * 8), gt);
     unpack8(*reinterpret_cast<const bf16x8*>(y1 + t * ld_y1 + F + v * 8), up);
 #pragma unroll
-    for (int k = 0; k < 8; ++k) {
-      const float sig = 1.f / (1.f + __expf(-gt[k]));
-      o[k] = gt[k] * sig * up[k];
-    }
+    for (int k = 0; k < 8; ++k) o[k] = swiglu_fwd_elem(gt[k], up[k]);
     *reinterpret_cast<bf16x8*>(act + t * ld_act + v * 8) = pack8(o);
   }
 }

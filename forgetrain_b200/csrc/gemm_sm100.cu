@@ -142,14 +142,6 @@ __device__ __forceinline__ void tmem_ld_packed256(uint32_t taddr, float alpha, u
   }
 }
 
-// silu(gate) * up of two packed bf16 pairs, the arithmetic of swiglu_fwd_kernel.
-__device__ __forceinline__ uint32_t swiglu_pair(uint32_t gw, uint32_t uw) {
-  const float g0 = __uint_as_float(gw << 16), g1 = __uint_as_float(gw & 0xffff0000u);
-  const float u0 = __uint_as_float(uw << 16), u1 = __uint_as_float(uw & 0xffff0000u);
-  const float s0 = 1.f / (1.f + __expf(-g0)), s1 = 1.f / (1.f + __expf(-g1));
-  return pack_bf16x2(g0 * s0 * u0, g1 * s1 * u1);
-}
-
 // Epilogue of one 128 x ncols accumulator for one warp: its 32 TMEM lanes (rows row0..row0+31),
 // column half `chalf`. TMEM -> registers -> (alpha, convert) -> swizzled staging buffer ->
 // TMA store / reduce-add. `nstores` counts this warp's bulk groups so the staging buffer is
@@ -284,7 +276,7 @@ __device__ __forceinline__ void drain_tile_swiglu(const GemmParams& p, const CUt
   release();
   store_piece(tmY, p.swiglu_F + gcol, row0, u, sbuf, lane, nstores);
 #pragma unroll
-  for (int i = 0; i < 32; ++i) g[i] = swiglu_pair(g[i], u[i]);
+  for (int i = 0; i < 32; i += 2) swiglu_fwd_pack4(g[i], g[i + 1], u[i], u[i + 1], g[i], g[i + 1]);
   store_piece(tmAct, gcol, row0, g, sbuf, lane, nstores);
 }
 
@@ -305,7 +297,8 @@ __device__ __forceinline__ void drain_tile_swiglu_whole(const GemmParams& p,
     const int gcol = n0 + c * 64;
     store_piece(tmY, gcol, row0, w + c * 32, sbuf, lane, nstores);
 #pragma unroll
-    for (int i = 0; i < 32; ++i) w[c * 32 + i] = swiglu_pair(w[c * 32 + i], w[64 + c * 32 + i]);
+    for (int i = c * 32; i < c * 32 + 32; i += 2)
+      swiglu_fwd_pack4(w[i], w[i + 1], w[64 + i], w[64 + i + 1], w[i], w[i + 1]);
     store_piece(tmY, p.swiglu_F + gcol, row0, w + 64 + c * 32, sbuf, lane, nstores);
     store_piece(tmAct, gcol, row0, w + c * 32, sbuf, lane, nstores);
   }
@@ -1391,11 +1384,19 @@ extern "C" int ft_gemm_swiglu_bf16(const void* A, const void* W, void* Y, void* 
   if (F % 128) return -2;
   const int sms = num_sms();
   if (max_ctas <= 0 || max_ctas > sms) max_ctas = sms;
-  // Two row blocks from K = 2048 on: 8B FC1 at 8192 tokens 1.75 -> 1.53 ms, at 4096 tokens 788 -> 751
-  // us. At K = 1024 a tile's main loop is shorter than the three stores and the activation of its
-  // 256 x 128 outputs take the four warps of an accumulator: 253 -> 263 us at 16384 tokens.
   const int k_iters = (K + GEMM_BK - 1) / GEMM_BK;
-  const int mt = k_iters >= 32 && pick_plan(M, 2 * F, k_iters, 0, 0, max_ctas).mt == 2 ? 2 : 1;
+  // Two row blocks where the schedule is shorter by pick_plan's units; the three stores and the
+  // activations of a row block add about 3 k-steps to a tile and 2 to the schedule, and the tail of
+  // the 128-row tiles is not cut here. us with one -> two: 0.5B at 1024 tokens 21.0 -> 23.7 (one is
+  // taken), 4096 61.8 -> 61.7, 8192 121 -> 116, 16384 241 -> 228; 8B at 8192 tokens 1750 -> 1532 (both
+  // with the divided activation).
+  const long tiles1 = static_cast<long>((M + GEMM_BM - 1) / GEMM_BM) * (F / 128);
+  const long tiles2 = static_cast<long>((M + 2 * GEMM_BM - 1) / (2 * GEMM_BM)) * (F / 128);
+  const long rem2 = tiles2 % max_ctas;
+  const long cost1 = (tiles1 + max_ctas - 1) / max_ctas * 100 * k_iters;
+  const long cost2 = tiles2 / max_ctas * (175 * k_iters + 300) +
+                     (rem2 == 0 ? 0 : 2 * rem2 <= max_ctas ? 120 * k_iters + 300 : 175 * k_iters + 300);
+  const int mt = cost2 + cost2 / 50 + 200 < cost1 ? 2 : 1;
   GemmParams p;
   p.M = M; p.N = 2 * F; p.K = K;
   p.a_mn = 0; p.b_mn = 0;

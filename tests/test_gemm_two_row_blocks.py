@@ -79,3 +79,16 @@ def test_fc1_swiglu_with_two_row_blocks_is_bitwise_the_two_kernels(T, F, K):
     y, act = gemm.linear_swiglu_fwd(x, w)
     assert torch.equal(y, gemm.linear_fwd(x, w, bn=256))
     assert torch.equal(act, cuda_ops.swiglu_fwd(y))
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("scale", [0.02, 0.3, 4.0])
+@pytest.mark.parametrize("T,F,K", [(128, 128, 64), (1000, 1024, 256), (2560, 8192, 2048)])
+def test_fused_activation_is_bitwise_the_divided_one_for_small_and_huge_gates(T, F, K, scale):
+    """Gates up to several hundred in magnitude (underflowing and saturated sigmoids), millions of values:
+    those near the middle of two bf16 numbers have to take the divided form."""
+    from forgetrain_b200.ops import cuda_ops, gemm
+    x = torch.randn(T, K, device="cuda").to(torch.bfloat16)
+    w = (torch.randn(2 * F, K, device="cuda") * scale).to(torch.bfloat16)
+    y, act = gemm.linear_swiglu_fwd(x, w)
+    assert torch.equal(act, cuda_ops.swiglu_fwd(y))
