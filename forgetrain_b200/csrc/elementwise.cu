@@ -174,7 +174,7 @@ rmsnorm_bwd_kernel(const __nv_bfloat16* __restrict__ dy, const __nv_bfloat16* __
   pdl_trigger();
   pdl_wait();
   __shared__ float red[4];
-  extern __shared__ float dw_smem[];  // [H] when TPR == 32 (cross-warp fold), unused otherwise
+  extern __shared__ __align__(16) float dw_smem[];  // [4][H] when TPR == 32 (cross-warp fold)
   constexpr int ROWS_PER_CTA = 128 / TPR;
   const int sub = threadIdx.x / TPR;
   const int tr = threadIdx.x % TPR;
@@ -257,14 +257,25 @@ rmsnorm_bwd_kernel(const __nv_bfloat16* __restrict__ dy, const __nv_bfloat16* __
       o4[1] = make_float4(acc[i][4], acc[i][5], acc[i][6], acc[i][7]);
     }
   } else {
-    for (int i = threadIdx.x; i < H; i += 128) dw_smem[i] = 0.f;
-    __syncthreads();
+    // a row of H sums per warp, then four columns per thread over the warps, in warp order
+    // (float atomics of all warps into one shared row cost 4 us: with the column sums, H = 1024, 512 / 2048 /
+    // 16384 tokens 8.5 -> 4.7, 11.7 -> 7.2, 31.9 -> 28.9 us)
+    float4* mine = reinterpret_cast<float4*>(dw_smem + warp * H);
 #pragma unroll
-    for (int i = 0; i < NV; ++i)
-#pragma unroll
-      for (int k = 0; k < 8; ++k) atomicAdd(&dw_smem[(tr + i * TPR) * 8 + k], acc[i][k]);
+    for (int i = 0; i < NV; ++i) {
+      mine[(tr + i * TPR) * 2] = make_float4(acc[i][0], acc[i][1], acc[i][2], acc[i][3]);
+      mine[(tr + i * TPR) * 2 + 1] = make_float4(acc[i][4], acc[i][5], acc[i][6], acc[i][7]);
+    }
     __syncthreads();
-    for (int i = threadIdx.x; i < H; i += 128) outp[i] = dw_smem[i];
+    for (int i = threadIdx.x; i < H / 4; i += 128) {
+      float4 a = reinterpret_cast<const float4*>(dw_smem)[i];
+#pragma unroll
+      for (int k = 1; k < 4; ++k) {
+        const float4 b = reinterpret_cast<const float4*>(dw_smem + k * H)[i];
+        a.x += b.x; a.y += b.y; a.z += b.z; a.w += b.w;
+      }
+      reinterpret_cast<float4*>(outp)[i] = a;
+    }
   }
 }
 
@@ -749,7 +760,7 @@ extern "C" int ft_rmsnorm_bwd(const void* dy, const void* h, const void* w, cons
   int nv, tpr;
   if (!norm_cfg(H, &nv, &tpr)) return -1;
   const int grid = ft_rmsnorm_bwd_partials(T, H);
-  const size_t smem = tpr == 32 ? (size_t)H * 4 : 0;
+  const size_t smem = tpr == 32 ? (size_t)H * 16 : 0;
 #define CALL_BWD                                                                          \
   launch_pdl(rmsnorm_bwd_kernel<NV, TPR>, grid, 128, smem, st,                                    \
       (const __nv_bfloat16*)dy, (const __nv_bfloat16*)h, (const __nv_bfloat16*)w,         \
@@ -890,7 +901,7 @@ extern "C" int ft_rmsnorm_bwd_noalloc(const void* dy, const void* h, const void*
   const int rows_per_cta = 128 / tpr;
   long want = (static_cast<long>(T) + rows_per_cta - 1) / rows_per_cta;
   const int grid = want < 1 ? 1 : (want > FT_NOALLOC_MAX_PARTIALS ? FT_NOALLOC_MAX_PARTIALS : (int)want);
-  const size_t smem = tpr == 32 ? (size_t)H * 4 : 0;
+  const size_t smem = tpr == 32 ? (size_t)H * 16 : 0;
 #define CALL_BWD_NA                                                                       \
   launch_pdl(rmsnorm_bwd_kernel<NV, TPR>, grid, 128, smem, st,                                    \
       (const __nv_bfloat16*)dy, (const __nv_bfloat16*)h, (const __nv_bfloat16*)w,         \
