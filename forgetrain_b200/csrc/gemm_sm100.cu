@@ -67,11 +67,12 @@ struct GemmParams {
   int ldd;
 };
 
-// MT: 128-row blocks of A per tile (1: 128 x BN tiles, 2: 256 x BN tiles)
-template <int BN, int STAGES, int EPI_BUFS = 1, int MT = 1>
+// MT: 128-row blocks of A per tile (1: 128 x BN tiles, 2: 256 x BN tiles); KB: boxes of 64 along the
+// reduction per stage (and per k-step)
+template <int BN, int STAGES, int EPI_BUFS = 1, int MT = 1, int KB = 1>
 struct GemmSmem {
-  static constexpr int A_BYTES = MT * GEMM_BM * GEMM_BK * 2;
-  static constexpr int B_BYTES = BN * GEMM_BK * 2;
+  static constexpr int A_BYTES = MT * GEMM_BM * GEMM_BK * 2 * KB;
+  static constexpr int B_BYTES = BN * GEMM_BK * 2 * KB;
   static constexpr int STAGE_BYTES = A_BYTES + B_BYTES;
   static constexpr int EPI_BUF_BYTES = 4096 * EPI_BUFS;      // boxes of 32 rows x 128 B
   static constexpr int EPI_BYTES = GEMM_EPI_WARPS * EPI_BUF_BYTES;  // one buffer per warp
@@ -170,8 +171,10 @@ __device__ __forceinline__ void drain_tile(const GemmParams& p, const CUtensorMa
     return;
   }
   if (p.out_mode == OUT_BF16) {
+    // 64-column pieces; of a 64-column tile's single one the first of the two warps takes care
+    const int per = max(1, ncols / 128);
 #pragma unroll 1
-    for (int c = chalf * (ncols / 128); c < (chalf + 1) * (ncols / 128); ++c) {
+    for (int c = chalf * per; c < min((chalf + 1) * per, ncols / 64); ++c) {
       const int col0 = colbase + c * 64;
       if (col0 >= p.N || !rows_live) break;
       uint32_t r[64];
@@ -420,7 +423,11 @@ __device__ __forceinline__ void swiglu_bwd_tile_info(const GemmParams& p, int ti
 // 512 tensor cycles (96 B per cycle and SM, above the ~75 that arrive from L2), a 256 x 256 tile
 // 64 KB per 1024 cycles. `it` counts accumulators, so that buffer and phase of block s of a unit are
 // (it + s) & 1 and ((it + s) >> 1) & 1 in the issuing and in the epilogue warps alike.
-template <int BN, int STAGES, int EPI = EPI_PLAIN, int MT = 1>
+//
+// KB == 2 (128 x 64 tiles, for narrow outputs of few tokens): a stage holds 128 of the reduction. With
+// one box of each operand per stage the tile asks for 24 KB at a time, and the two producer warps,
+// each held about 400 cycles by an issue, bring a stage every 420 cycles whatever its size.
+template <int BN, int STAGES, int EPI = EPI_PLAIN, int MT = 1, int KB = 1>
 __global__ void __launch_bounds__(GEMM_THREADS, 1)
 gemm_bf16_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUtensorMap tmB,
                  const __grid_constant__ CUtensorMap tmD, const __grid_constant__ CUtensorMap tmD2,
@@ -431,7 +438,8 @@ gemm_bf16_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant_
                 "the fused SwiGLU epilogues are built for 256-column tiles");
   static_assert(MT == 1 || (MT == 2 && BN == 256 && EPI != EPI_SWIGLU_BWD),
                 "two row blocks: 256-column tiles, and one staging buffer per epilogue warp");
-  using L = GemmSmem<BN, STAGES, EPI == EPI_SWIGLU_BWD ? 2 : 1, MT>;
+  static_assert(KB == 1 || (BN == 64 && MT == 1 && EPI == EPI_PLAIN), "built for 128 x 64 tiles");
+  using L = GemmSmem<BN, STAGES, EPI == EPI_SWIGLU_BWD ? 2 : 1, MT, KB>;
   extern __shared__ uint8_t smem_raw[];
   uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) &
                                              ~static_cast<uintptr_t>(1023));
@@ -489,8 +497,10 @@ gemm_bf16_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant_
     // (MN-major) per row block; B is BN/128 boxes of 128 rows or BN/64 boxes of 64 x 64.
     const int pid = warp == 0 ? 0 : 1;
     const int nA = (p.a_mn ? GEMM_BM / 64 : 1) * MT;
-    const int nB = p.b_mn ? BN / 64 : BN / 128;
-    if (lane < nA + nB) {
+    const int nB = p.b_mn ? BN / 64 : (BN + 127) / 128;
+    const int kbox = lane / (nA + nB);           // which 64 of the stage's reduction
+    const int box = lane - kbox * (nA + nB);     // which box of those
+    if (kbox < KB) {
       int stage = 0;
       uint32_t phase = 0;
       for (int tile = unit0; tile < total_tiles; tile += ustep) {
@@ -508,29 +518,27 @@ gemm_bf16_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant_
         for (int ki = kb; ki < kb + kn; ++ki) {
           if ((stage & 1) == pid) {
             mbar_wait(&empty_bar[stage], phase ^ 1, abort_flag, p.status, FT_ERR_WAIT_EMPTY);
-            uint8_t* sA = smem + stage * L::STAGE_BYTES;
-            uint8_t* sB = sA + L::A_BYTES;
+            uint8_t* sA = smem + stage * L::STAGE_BYTES + kbox * (L::A_BYTES / KB);
+            uint8_t* sB = smem + stage * L::STAGE_BYTES + L::A_BYTES + kbox * (L::B_BYTES / KB);
+            const int kx = (ki * KB + kbox) * GEMM_BK;
             if (lane == 0) mbar_expect_tx(&full_bar[stage], tx);
-            if (lane < nA) {
-              if (lane < nAt) {
+            if (box < nA) {
+              if (box < nAt) {
                 if (!p.a_mn)
-                  tma_load_2d(sA + lane * 16384, &tmA, &full_bar[stage], ki * GEMM_BK,
-                              row0 + lane * GEMM_BM);
+                  tma_load_2d(sA + box * 16384, &tmA, &full_bar[stage], kx, row0 + box * GEMM_BM);
                 else
-                  tma_load_2d(sA + lane * 8192, &tmA, &full_bar[stage], row0 + lane * 64,
-                              ki * GEMM_BK);
+                  tma_load_2d(sA + box * 8192, &tmA, &full_bar[stage], row0 + box * 64, kx);
               }
-            } else if (lane - nA < nBt) {
-              const int j = lane - nA;           // slot in the B buffer; jb0 + j: box of the tile
+            } else if (box - nA < nBt) {
+              const int j = box - nA;            // slot in the B buffer; jb0 + j: box of the tile
               if (SWIGLU)   // box 0: 128 gate rows, box 1: the 128 up rows of the same columns
-                tma_load_2d(sB + j * 16384, &tmB, &full_bar[stage], ki * GEMM_BK,
+                tma_load_2d(sB + j * 16384, &tmB, &full_bar[stage], kx,
                             nt * 128 + j * p.swiglu_F);
               else if (!p.b_mn)
-                tma_load_2d(sB + j * 16384, &tmB, &full_bar[stage], ki * GEMM_BK,
+                tma_load_2d(sB + j * 16384, &tmB, &full_bar[stage], kx,
                             nt * BN + (jb0 + j) * 128);
               else
-                tma_load_2d(sB + j * 8192, &tmB, &full_bar[stage], nt * BN + (jb0 + j) * 64,
-                            ki * GEMM_BK);
+                tma_load_2d(sB + j * 8192, &tmB, &full_bar[stage], nt * BN + (jb0 + j) * 64, kx);
             }
           }
           if (++stage == STAGES) { stage = 0; phase ^= 1; }
@@ -633,8 +641,11 @@ gemm_bf16_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant_
             const uint32_t b_lo = smem_desc_lo(sA + L::A_BYTES, b_lbo);
             umma_ss_lo_dyn(tmem_d, a_lo, b_lo, idesc, ki > 0 ? 1u : 0u);
 #pragma unroll
-            for (int kk = 1; kk < GEMM_BK / 16; ++kk)
-              umma_ss_lo<1>(tmem_d, a_lo + kk * a_kstep, b_lo + kk * b_kstep, idesc);
+            for (int kk = 1; kk < KB * (GEMM_BK / 16); ++kk) {
+              const int kb4 = kk / (GEMM_BK / 16), k4 = kk % (GEMM_BK / 16);
+              umma_ss_lo<1>(tmem_d, a_lo + kb4 * ((L::A_BYTES / KB) >> 4) + k4 * a_kstep,
+                            b_lo + kb4 * ((L::B_BYTES / KB) >> 4) + k4 * b_kstep, idesc);
+            }
             umma_commit(&empty_bar[stage]);
           }
           __syncwarp();
@@ -1113,14 +1124,14 @@ static int num_sms() {
   return g_num_sms;
 }
 
-template <int BN, int STAGES, int EPI = EPI_PLAIN, int MT = 1>
+template <int BN, int STAGES, int EPI = EPI_PLAIN, int MT = 1, int KB = 1>
 static int launch_gemm(const CUtensorMap& tmA, const CUtensorMap& tmB, const CUtensorMap& tmD,
                        const CUtensorMap& tmD2, const GemmParams& p, int max_ctas,
                        cudaStream_t stream) {
-  using L = GemmSmem<BN, STAGES, EPI == EPI_SWIGLU_BWD ? 2 : 1, MT>;
+  using L = GemmSmem<BN, STAGES, EPI == EPI_SWIGLU_BWD ? 2 : 1, MT, KB>;
   static bool attr_set = false;
   if (!attr_set) {
-    cudaError_t e = cudaFuncSetAttribute(gemm_bf16_kernel<BN, STAGES, EPI, MT>,
+    cudaError_t e = cudaFuncSetAttribute(gemm_bf16_kernel<BN, STAGES, EPI, MT, KB>,
                                          cudaFuncAttributeMaxDynamicSharedMemorySize, L::TOTAL);
     if (e != cudaSuccess) return -10;
     attr_set = true;
@@ -1128,7 +1139,7 @@ static int launch_gemm(const CUtensorMap& tmA, const CUtensorMap& tmB, const CUt
   const int total = p.total_units;
   int grid = total < max_ctas || EPI == EPI_CLUSTER ? total : max_ctas;
   if (grid < 1) grid = 1;
-  launch_pdl_cluster(gemm_bf16_kernel<BN, STAGES, EPI, MT>, EPI == EPI_CLUSTER ? p.splitk : 1, grid,
+  launch_pdl_cluster(gemm_bf16_kernel<BN, STAGES, EPI, MT, KB>, EPI == EPI_CLUSTER ? p.splitk : 1, grid,
                      GEMM_THREADS, L::TOTAL, stream, tmA, tmB, tmD, tmD2, p);
   return cudaGetLastError() == cudaSuccess ? 0 : -11;
 }
@@ -1207,6 +1218,9 @@ static int max_clusters(int size) {
 //     fc1 dgrad  2048 x 1024 x 8192   40.8 -> 36.2                     8B fc1 dgrad 256 x 4096 x 32768  156 -> 118 -> 73
 //     wo dgrad    256 x 1024 x 1024    7.0 ->  6.9 ->  6.8 (S = 4)
 //   A cluster costs its launch, two barriers and the exchange: 3.5 us, 9 k-steps.
+//   128 x 128 -> 128 x 64 tiles with two boxes per stage (0.46; with one box 0.6), bf16 results, when they all run
+//   at once: fc2 fwd 512 x 1024 x 4096 18.0 -> 14.7, qkv fwd 512 x 1280 x 1024 7.4 -> 6.2, wo dgrad 1024 x 1024 x
+//   1024 7.9 -> 6.8, 8B fc2 fwd 256 x 4096 x 16384 62 -> 52; 160 of them (qkv fwd, 1024 tokens) 8.0 -> 9.3.
 //   fp32 results: splitting over the grid costs the memset and the reduce-adds, 16.5 k-steps, or 7
 //   into a gradient that is accumulated anyway (wo wgrad 1024 x 1024 x T, T = 2048: 128 x 128 12.4,
 //   cluster of two 11.5, grid split in four 13.2; accumulating 12.6, 13.2, 10.4).
@@ -1242,6 +1256,7 @@ static GemmPlan pick_plan(int M, int N, int k_iters, int kind, int accumulate, i
       offer(GemmPlan{mt, 256, s, 1}, cost);
     }
   }
+  if (!f32 && mt128 * ((N + 63) / 64) <= max_ctas) offer(GemmPlan{1, 64, 1, 1}, 46L * k_iters);
   const long tiles = mt128 * ((N + 127) / 128);
   if (tiles <= max_ctas) {   // with more tiles the wider ones load less per product
     // fp32: through the cluster kernel, with its four accumulators, also without a cluster
@@ -1302,7 +1317,7 @@ static int launch_gemm_pair(const CUtensorMap& tmA, const CUtensorMap& tmB,
 //   [K][lda] (row index contiguous). Same for B with N. out_dtype: 0 bf16, 1 fp32.
 //   accumulate != 0 (fp32 only): D += result. splitk <= 0 picks a split automatically
 //   (fp32 only); bn in {0 (auto), 128, 256: one 128 x bn tile, 512: a 256 x 256 tile per CTA,
-//   1000 + S: 128 x 128 tiles whose reduction is split inside clusters of S = 2 .. 8 CTAs}. All leading dimensions in elements; every base
+//   64 (bf16 only): 128 x 64 tiles, 1000 + S: 128 x 128 tiles whose reduction is split inside clusters of S = 2 .. 8 CTAs}. All leading dimensions in elements; every base
 //   pointer 16-byte aligned and every leading dimension a multiple of 8 (bf16) / 4 (fp32).
 extern "C" int ft_gemm_bf16(const void* A, const void* B, void* D, int M, int N, int K, int lda,
                             int ldb, int ldd, int a_mn, int b_mn, int out_dtype, int accumulate,
@@ -1314,16 +1329,18 @@ extern "C" int ft_gemm_bf16(const void* A, const void* B, void* D, int M, int N,
   if (out_dtype == 0 && accumulate) return -2;
   const int sms = num_sms();
   if (max_ctas <= 0 || max_ctas > sms) max_ctas = sms;
-  const int k_iters = (K + GEMM_BK - 1) / GEMM_BK;
+  int k_iters = (K + GEMM_BK - 1) / GEMM_BK;
   GemmPlan plan{bn == 512 ? 2 : 1, bn, splitk, 1};
   if (out_dtype == 0) splitk = plan.splitk = 1;
-  const bool given = bn == 128 || bn == 256 || bn == 512;
+  const bool narrow = bn == 64 && out_dtype == 0;
+  const bool given = narrow || bn == 128 || bn == 256 || bn == 512;
   if (bn != 128 && bn != 256) bn = (N <= 128) ? 128 : 256;
-  plan.bn = bn;
+  plan.bn = narrow ? 64 : bn;
   if (cluster > 0) plan = GemmPlan{1, 128, 1, cluster == 1 ? -1 : cluster < k_iters ? cluster : k_iters};
   else if (!given && N > 128 && (out_dtype == 0 || splitk <= 0))
     plan = pick_plan(M, N, k_iters, out_dtype == 1 ? 2 : b_mn ? 1 : 0, accumulate, max_ctas);
   bn = plan.bn;
+  if (bn == 64) k_iters = (K + 2 * GEMM_BK - 1) / (2 * GEMM_BK);   // two boxes per k-step
   const int mt = plan.mt;
   const int m_tiles = (M + GEMM_BM * mt - 1) / (GEMM_BM * mt);
   const int n_tiles = (N + bn - 1) / bn;
@@ -1358,7 +1375,7 @@ extern "C" int ft_gemm_bf16(const void* A, const void* B, void* D, int M, int N,
   if (!a_mn) rc = get_tmap_2d(&tmA, A, 2, M, K, lda, GEMM_BM, GEMM_BK);
   else       rc = get_tmap_2d(&tmA, A, 2, K, M, lda, GEMM_BK, 64);
   if (rc) return -4;
-  if (!b_mn) rc = get_tmap_2d(&tmB, B, 2, N, K, ldb, 128, GEMM_BK);
+  if (!b_mn) rc = get_tmap_2d(&tmB, B, 2, N, K, ldb, bn == 64 ? 64 : 128, GEMM_BK);
   else       rc = get_tmap_2d(&tmB, B, 2, K, N, ldb, GEMM_BK, 64);
   if (rc) return -5;
   if (out_dtype == 0) rc = get_tmap_2d(&tmD, D, 2, M, N, ldd, 32, 64);
@@ -1369,6 +1386,8 @@ extern "C" int ft_gemm_bf16(const void* A, const void* B, void* D, int M, int N,
     return launch_gemm<128, 6, EPI_CLUSTER>(tmA, tmB, tmD, tmD, p, max_ctas, stream);
   if (mt == 2) return launch_gemm<256, 3, EPI_PLAIN, 2>(tmA, tmB, tmD, tmD, p, max_ctas, stream);
   if (bn == 256) return launch_gemm<256, 4>(tmA, tmB, tmD, tmD, p, max_ctas, stream);
+  if (bn == 64)
+    return launch_gemm<64, 4, EPI_PLAIN, 1, 2>(tmA, tmB, tmD, tmD, p, max_ctas, stream);
   return launch_gemm<128, 6>(tmA, tmB, tmD, tmD, p, max_ctas, stream);
 }
 

@@ -63,3 +63,16 @@ def test_split_reductions_are_no_less_exact_and_the_forward_pass_is_not_split(T,
     assert torch.equal(gemm.linear_fwd(dy, wt), gemm.linear_fwd(dy, wt, bn=256))
     # a row of the forward result does not depend on how many rows there are
     assert torch.equal(gemm.linear_fwd(dy, wt)[:128], gemm.linear_fwd(dy[:128], wt))
+
+
+# rows / columns that end inside a tile, an odd number of 64-wide boxes, a partial one, fewer k-steps than stages
+@pytest.mark.gpu
+@pytest.mark.parametrize("T,N,K", [(128, 64, 64), (200, 72, 192), (384, 328, 128), (512, 1280, 1024), (130, 136, 1000),
+                                   (136, 1288, 4096)])
+def test_narrow_tiles_are_bitwise_the_wide_ones(T, N, K):
+    from forgetrain_b200.ops import gemm
+    x = torch.randn(T, K, device="cuda").to(torch.bfloat16)
+    w = (torch.randn(N, K, device="cuda") * 0.05).to(torch.bfloat16)
+    assert torch.equal(gemm.linear_fwd(x, w, alpha=0.5, bn=64), gemm.linear_fwd(x, w, alpha=0.5, bn=256))
+    w2 = (torch.randn(K, N, device="cuda") * 0.05).to(torch.bfloat16)
+    assert torch.equal(gemm.linear_dgrad(x, w2, bn=64), gemm.linear_dgrad(x, w2, bn=256))
