@@ -283,6 +283,40 @@ __device__ __forceinline__ void drain_tile_swiglu(const GemmParams& p, const CUt
   store_piece(tmAct, gcol, row0, g, sbuf, lane, nstores);
 }
 
+// The same for a 128-column tile (64 gate columns and the matching 64 up columns): both warps of a lane
+// quarter read everything, one writes the gate and the activation, the other the up columns.
+template <class Release>
+__device__ __forceinline__ void drain_tile_swiglu_narrow(const GemmParams& p,
+                                                         const CUtensorMap* tmY,
+                                                         const CUtensorMap* tmAct, uint32_t taddr,
+                                                         int row0, int gcol, int chalf,
+                                                         uint8_t* sbuf, int lane, int& nstores,
+                                                         Release release) {
+  uint32_t w[64];   // 64 gate, then 64 up values of this thread's row, packed bf16x2
+#pragma unroll
+  for (int c = 0; c < 2; ++c) {
+    uint32_t r[64];
+    tmem_ld32(taddr + c * 64, r);
+    tmem_ld32(taddr + c * 64 + 32, r + 32);
+    tmem_ld_wait();
+#pragma unroll
+    for (int i = 0; i < 32; ++i)
+      w[c * 32 + i] = pack_bf16x2(__uint_as_float(r[2 * i]) * p.alpha,
+                                  __uint_as_float(r[2 * i + 1]) * p.alpha);
+  }
+  release();
+  if (row0 >= p.M || gcol >= p.swiglu_F) return;
+  if (chalf == 1) {
+    store_piece(tmY, p.swiglu_F + gcol, row0, w + 32, sbuf, lane, nstores);
+    return;
+  }
+  store_piece(tmY, gcol, row0, w, sbuf, lane, nstores);
+#pragma unroll
+  for (int i = 0; i < 32; i += 2)
+    swiglu_fwd_pack4(w[i], w[i + 1], w[32 + i], w[32 + i + 1], w[i], w[i + 1]);
+  store_piece(tmAct, gcol, row0, w, sbuf, lane, nstores);
+}
+
 // The same for a tile of two row blocks (see WHOLE at drain_tile): one warp drains the gate and
 // the up columns of its 32 rows, all of them into registers first.
 template <class Release>
@@ -434,8 +468,8 @@ gemm_bf16_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant_
                  const GemmParams p) {
   pdl_trigger();
   constexpr bool SWIGLU = EPI == EPI_SWIGLU_FWD;
-  static_assert(EPI == EPI_PLAIN || EPI == EPI_CLUSTER || BN == 256,
-                "the fused SwiGLU epilogues are built for 256-column tiles");
+  static_assert(EPI != EPI_SWIGLU_BWD || BN == 256, "built for 256-column tiles");
+  static_assert(EPI != EPI_SWIGLU_FWD || BN == 256 || (BN == 128 && MT == 1), "gate and up halves");
   static_assert(MT == 1 || (MT == 2 && BN == 256 && EPI != EPI_SWIGLU_BWD),
                 "two row blocks: 256-column tiles, and one staging buffer per epilogue warp");
   static_assert(KB == 1 || (BN == 64 && MT == 1 && EPI == EPI_PLAIN), "built for 128 x 64 tiles");
@@ -497,7 +531,7 @@ gemm_bf16_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant_
     // (MN-major) per row block; B is BN/128 boxes of 128 rows or BN/64 boxes of 64 x 64.
     const int pid = warp == 0 ? 0 : 1;
     const int nA = (p.a_mn ? GEMM_BM / 64 : 1) * MT;
-    const int nB = p.b_mn ? BN / 64 : (BN + 127) / 128;
+    const int nB = SWIGLU ? 2 : p.b_mn ? BN / 64 : (BN + 127) / 128;
     const int kbox = lane / (nA + nB);           // which 64 of the stage's reduction
     const int box = lane - kbox * (nA + nB);     // which box of those
     if (kbox < KB) {
@@ -531,9 +565,9 @@ gemm_bf16_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant_
               }
             } else if (box - nA < nBt) {
               const int j = box - nA;            // slot in the B buffer; jb0 + j: box of the tile
-              if (SWIGLU)   // box 0: 128 gate rows, box 1: the 128 up rows of the same columns
-                tma_load_2d(sB + j * 16384, &tmB, &full_bar[stage], kx,
-                            nt * 128 + j * p.swiglu_F);
+              if (SWIGLU)   // box 0: BN / 2 gate rows, box 1: the up rows of the same columns
+                tma_load_2d(sB + j * (BN * 64), &tmB, &full_bar[stage], kx,
+                            nt * (BN / 2) + j * p.swiglu_F);
               else if (!p.b_mn)
                 tma_load_2d(sB + j * 16384, &tmB, &full_bar[stage], kx,
                             nt * BN + (jb0 + j) * 128);
@@ -806,6 +840,9 @@ gemm_bf16_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant_
         else if (SWIGLU && MT == 2)
           drain_tile_swiglu_whole(p, &tmD, &tmD2, taddr, row0, nt * 128, my_epi, lane, nstores,
                                   release);
+        else if (SWIGLU && BN == 128)
+          drain_tile_swiglu_narrow(p, &tmD, &tmD2, taddr, row0, nt * 64, chalf, my_epi, lane,
+                                   nstores, release);
         else if (SWIGLU)
           drain_tile_swiglu(p, &tmD, &tmD2, taddr, row0, nt * 128, chalf, my_epi, lane, nstores,
                             release);
@@ -1416,6 +1453,9 @@ extern "C" int ft_gemm_swiglu_bf16(const void* A, const void* W, void* Y, void* 
   const long cost2 = tiles2 / max_ctas * (175 * k_iters + 300) +
                      (rem2 == 0 ? 0 : 2 * rem2 <= max_ctas ? 120 * k_iters + 300 : 175 * k_iters + 300);
   const int mt = cost2 + cost2 / 50 + 200 < cost1 ? 2 : 1;
+  // 64 gate and 64 up columns per tile while all tiles run at once: 0.5B at 256 tokens 13.8 -> 11.4 us, the
+  // tiny model at 512 tokens 8.1 -> 7.2 us.
+  const bool narrow = 2 * tiles1 <= max_ctas;
   GemmParams p;
   p.M = M; p.N = 2 * F; p.K = K;
   p.a_mn = 0; p.b_mn = 0;
@@ -1423,7 +1463,7 @@ extern "C" int ft_gemm_swiglu_bf16(const void* A, const void* W, void* Y, void* 
   p.alpha = alpha;
   p.splitk = 1;
   p.m_tiles = (M + GEMM_BM * mt - 1) / (GEMM_BM * mt);
-  p.n_tiles = F / 128;
+  p.n_tiles = narrow ? F / 64 : F / 128;
   p.k_iters = k_iters;
   p.status = status;
   p.swiglu_F = F;
@@ -1431,9 +1471,11 @@ extern "C" int ft_gemm_swiglu_bf16(const void* A, const void* W, void* Y, void* 
   if (mt == 2) cut_tail(p, max_ctas);
   CUtensorMap tmA, tmB, tmY, tmAct;
   if (get_tmap_2d(&tmA, A, 2, M, K, lda, GEMM_BM, GEMM_BK)) return -4;
-  if (get_tmap_2d(&tmB, W, 2, 2 * static_cast<uint64_t>(F), K, ldw, 128, GEMM_BK)) return -5;
+  if (get_tmap_2d(&tmB, W, 2, 2 * static_cast<uint64_t>(F), K, ldw, narrow ? 64 : 128, GEMM_BK))
+    return -5;
   if (get_tmap_2d(&tmY, Y, 2, M, 2 * static_cast<uint64_t>(F), ldy, 32, 64)) return -6;
   if (get_tmap_2d(&tmAct, ACT, 2, M, F, ldact, 32, 64)) return -6;
+  if (narrow) return launch_gemm<128, 6, EPI_SWIGLU_FWD>(tmA, tmB, tmY, tmAct, p, max_ctas, stream);
   if (mt == 2)
     return launch_gemm<256, 3, EPI_SWIGLU_FWD, 2>(tmA, tmB, tmY, tmAct, p, max_ctas, stream);
   return launch_gemm<256, 4, EPI_SWIGLU_FWD>(tmA, tmB, tmY, tmAct, p, max_ctas, stream);

@@ -92,3 +92,15 @@ def test_fused_activation_is_bitwise_the_divided_one_for_small_and_huge_gates(T,
     w = (torch.randn(2 * F, K, device="cuda") * scale).to(torch.bfloat16)
     y, act = gemm.linear_swiglu_fwd(x, w)
     assert torch.equal(act, cuda_ops.swiglu_fwd(y))
+
+
+# 64 gate + 64 up columns per tile: a row block that ends inside a tile, one tile, as many as there are CTAs at most
+@pytest.mark.gpu
+@pytest.mark.parametrize("T,F,K", [(128, 128, 64), (200, 1024, 264), (256, 4096, 1024), (1100, 1024, 256)])
+def test_narrow_fc1_swiglu_is_bitwise_the_two_kernels(T, F, K):
+    from forgetrain_b200.ops import cuda_ops, gemm
+    x = torch.randn(T, K, device="cuda").to(torch.bfloat16)
+    w = (torch.randn(2 * F, K, device="cuda") * 0.1).to(torch.bfloat16)
+    y, act = gemm.linear_swiglu_fwd(x, w, alpha=0.5)
+    assert torch.equal(y, gemm.linear_fwd(x, w, alpha=0.5, bn=256))
+    assert torch.equal(act, cuda_ops.swiglu_fwd(y))
