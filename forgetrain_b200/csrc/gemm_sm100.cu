@@ -375,49 +375,63 @@ __device__ __forceinline__ void stage_partial(uint32_t taddr, int kn, uint8_t* s
   }
 }
 
-template <int BN>
+// NC: CTAs of the cluster. Every load of up to eight rows of a warp is issued before the first is
+// used: one row at a time the latencies of an exchange and of an accumulated output add up (NC = 1,
+// 16 rows per warp, accumulating: 7 us), one CTA at a time those of NC exchanges (NC = 6: 2.4 us).
+template <int BN, int NC>
 __device__ __forceinline__ void sum_partials(const GemmParams& p, const uint8_t* smem, int row0,
                                              int col0, int warp, int lane) {
   static_assert(BN == 128, "a lane takes four columns of a row");
-  const int ncta = p.splitk;
-  const int per = (GEMM_BM + ncta - 1) / ncta;
-  const int first = static_cast<int>(cluster_ctarank()) * per;
-  const int last = min(first + per, GEMM_BM);
+  constexpr int PER = (GEMM_BM + NC - 1) / NC;                       // rows of a CTA
+  constexpr int PER_WARP = (PER + GEMM_EPI_WARPS - 1) / GEMM_EPI_WARPS;
+  constexpr int ROWS = PER_WARP < 8 ? PER_WARP : 8;
+  const int first = (NC == 1 ? 0 : static_cast<int>(cluster_ctarank())) * PER;
+  const int last = min(first + PER, GEMM_BM);
   const int col = col0 + lane * 4;
-  for (int r = first + warp; r < last; r += GEMM_EPI_WARPS) {
-    const uint32_t at = smem_u32(smem) + (r * (BN + 4) + lane * 4) * 4;
-    float4 v[8];
+  for (int r0 = first + warp; r0 < last; r0 += ROWS * GEMM_EPI_WARPS) {
+    float4 v[ROWS][NC], o[ROWS];
 #pragma unroll
-    for (int c = 0; c < 8; ++c)
-      if (c < ncta) v[c] = ld_cluster_f4(mapa_u32(at, c));
-    float4 a = v[0];
+    for (int i = 0; i < ROWS; ++i) {
+      const int r = r0 + i * GEMM_EPI_WARPS, row = row0 + r;
+      o[i] = make_float4(0.f, 0.f, 0.f, 0.f);
+      if (p.out_mode == OUT_F32_ADD && r < last && row < p.M && col + 4 <= p.N)
+        o[i] = *reinterpret_cast<const float4*>(static_cast<const float*>(p.d) +
+                                                static_cast<long>(row) * p.ldd + col);
+      // past the end: some row of this CTA's own partial, which is read and not used
+      const uint32_t at = smem_u32(smem) + (min(r, GEMM_BM - 1) * (BN + 4) + lane * 4) * 4;
 #pragma unroll
-    for (int c = 1; c < 8; ++c)
-      if (c < ncta) { a.x += v[c].x; a.y += v[c].y; a.z += v[c].z; a.w += v[c].w; }
-    a.x *= p.alpha; a.y *= p.alpha; a.z *= p.alpha; a.w *= p.alpha;
-    const int row = row0 + r;
-    if (row >= p.M || col >= p.N) continue;
-    const long off = static_cast<long>(row) * p.ldd + col;
-    if (p.out_mode == OUT_BF16) {
-      __nv_bfloat16* d = static_cast<__nv_bfloat16*>(p.d) + off;
-      if (col + 4 <= p.N) {
-        *reinterpret_cast<uint2*>(d) = make_uint2(pack_bf16x2(a.x, a.y), pack_bf16x2(a.z, a.w));
-      } else {
-        const float e[3] = {a.x, a.y, a.z};
-        for (int i = 0; i < p.N - col; ++i) d[i] = __float2bfloat16_rn(e[i]);
+      for (int c = 0; c < NC; ++c)
+        v[i][c] = ld_cluster_f4(NC == 1 || r >= last ? mapa_u32(at, cluster_ctarank())
+                                                     : mapa_u32(at, c));
+    }
+#pragma unroll
+    for (int i = 0; i < ROWS; ++i) {
+      const int r = r0 + i * GEMM_EPI_WARPS, row = row0 + r;
+      if (r >= last || row >= p.M || col >= p.N) continue;
+      float4 q = v[i][0];
+#pragma unroll
+      for (int c = 1; c < NC; ++c) {
+        q.x += v[i][c].x; q.y += v[i][c].y; q.z += v[i][c].z; q.w += v[i][c].w;
       }
-    } else {
-      float* d = static_cast<float*>(p.d) + off;
-      if (col + 4 <= p.N) {
-        float4* d4 = reinterpret_cast<float4*>(d);
-        if (p.out_mode == OUT_F32_ADD) {
-          const float4 o = *d4;
-          a.x += o.x; a.y += o.y; a.z += o.z; a.w += o.w;
+      q = make_float4(q.x * p.alpha + o[i].x, q.y * p.alpha + o[i].y, q.z * p.alpha + o[i].z,
+                      q.w * p.alpha + o[i].w);
+      const long off = static_cast<long>(row) * p.ldd + col;
+      if (p.out_mode == OUT_BF16) {
+        __nv_bfloat16* d = static_cast<__nv_bfloat16*>(p.d) + off;
+        if (col + 4 <= p.N) {
+          *reinterpret_cast<uint2*>(d) = make_uint2(pack_bf16x2(q.x, q.y), pack_bf16x2(q.z, q.w));
+        } else {
+          const float e[3] = {q.x, q.y, q.z};
+          for (int k = 0; k < p.N - col; ++k) d[k] = __float2bfloat16_rn(e[k]);
         }
-        *d4 = a;
       } else {
-        const float e[3] = {a.x, a.y, a.z};
-        for (int i = 0; i < p.N - col; ++i) d[i] = p.out_mode == OUT_F32_ADD ? d[i] + e[i] : e[i];
+        float* d = static_cast<float*>(p.d) + off;
+        if (col + 4 <= p.N) {
+          *reinterpret_cast<float4*>(d) = q;
+        } else {
+          const float e[3] = {q.x, q.y, q.z};
+          for (int k = 0; k < p.N - col; ++k) d[k] = p.out_mode == OUT_F32_ADD ? d[k] + e[k] : e[k];
+        }
       }
     }
   }
@@ -869,7 +883,17 @@ gemm_bf16_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant_
     if (warp >= 2 && warp < 2 + GEMM_EPI_WARPS && unit0 < total_tiles) {
       int mt, nt, kb, kn, half;
       decode_tile<MT>(p, unit0, mt, nt, kb, kn, half);
-      sum_partials<BN>(p, smem, mt * GEMM_BM, nt * BN, warp - 2, lane);
+      const int r0 = mt * GEMM_BM, c0 = nt * BN, w = warp - 2;
+      switch (p.splitk) {
+        case 1: sum_partials<BN, 1>(p, smem, r0, c0, w, lane); break;
+        case 2: sum_partials<BN, 2>(p, smem, r0, c0, w, lane); break;
+        case 3: sum_partials<BN, 3>(p, smem, r0, c0, w, lane); break;
+        case 4: sum_partials<BN, 4>(p, smem, r0, c0, w, lane); break;
+        case 5: sum_partials<BN, 5>(p, smem, r0, c0, w, lane); break;
+        case 6: sum_partials<BN, 6>(p, smem, r0, c0, w, lane); break;
+        case 7: sum_partials<BN, 7>(p, smem, r0, c0, w, lane); break;
+        default: sum_partials<BN, 8>(p, smem, r0, c0, w, lane); break;
+      }
     }
     cluster_sync_all();   // nobody leaves while another CTA still reads its partial
   }
@@ -1296,8 +1320,9 @@ static GemmPlan pick_plan(int M, int N, int k_iters, int kind, int accumulate, i
   if (!f32 && mt128 * ((N + 63) / 64) <= max_ctas) offer(GemmPlan{1, 64, 1, 1}, 46L * k_iters);
   const long tiles = mt128 * ((N + 127) / 128);
   if (tiles <= max_ctas) {   // with more tiles the wider ones load less per product
-    // fp32: through the cluster kernel, with its four accumulators, also without a cluster
-    if (!f32 || chains <= CLUSTER_ACCS) offer(GemmPlan{1, 128, 1, f32 ? -1 : 1}, 66L * k_iters);
+    // in one chain, or (fp32) through the cluster kernel with its four accumulators on one CTA
+    if (!f32 || chains == 1) offer(GemmPlan{1, 128, 1, 1}, 66L * k_iters);
+    else if (chains <= CLUSTER_ACCS) offer(GemmPlan{1, 128, 1, -1}, 66L * k_iters + 500);
     for (int c = 2; kind > 0 && c <= 8 && tiles * c <= max_ctas && 2 * c <= k_iters; ++c) {
       const long cost = 66L * ((k_iters + c - 1) / c) + 900;
       // asked only where it could win: the occupancy query runs once per cluster size
